@@ -118,7 +118,10 @@ int nwg_bfs(nwg_graph g, uint32_t root, int alpha, int beta, uint32_t* parents_h
 /* nwg_bfs over k roots with each root's parents copied to host row i of
  * parents_host (k * n entries, row i = roots[i]); replaces the per-source
  * loop of NWGraph's BFS benchmark (bench/bfs.cpp:106-141), which calls
- * bfs(graph, gx, source, num_bins, alpha, beta) once per source.  Two
+ * bfs(graph, gx, source, num_bins, alpha, beta) once per source.  On small
+ * graphs (at most 2^19 vertices) many roots traverse side by side, one block
+ * each, and their rows are copied a launch at a time (buffers of up to 128 MB
+ * are kept with the graph).  Otherwise two
  * traversals are in flight: root i + 1 runs on the device while root i's
  * parents cross to the host, so with pinned host memory a call costs about
  * k copies of n * 4 bytes rather than k copies plus k traversals (pageable
@@ -134,8 +137,9 @@ int nwg_bfs_roots(nwg_graph g, const uint32_t* roots, uint64_t k, int alpha, int
 int nwg_ws_create(nwg_graph g, nwg_bfs_ws* out);
 int nwg_ws_destroy(nwg_bfs_ws ws);
 
-/* Stream-ordered variant of nwg_bfs: enqueues the whole traversal (one CUDA
- * cooperative kernel launch, no host synchronisation) on `stream` (a cudaStream_t, NULL =
+/* Stream-ordered variant of nwg_bfs: enqueues the whole traversal (one
+ * kernel launch, cooperative unless the graph is small; no host
+ * synchronisation) on `stream` (a cudaStream_t, NULL =
  * legacy default stream) writing parents to the device array parents_dev.
  * At most one traversal per workspace may be in flight. */
 int nwg_bfs_async(nwg_bfs_ws ws, uint32_t root, int alpha, int beta, uint32_t* parents_dev, void* stream);
@@ -235,8 +239,10 @@ int nwg_msbfs_ex(nwg_msbfs_ws ws, const uint32_t* roots_host, uint32_t k, void* 
  * (graph, root) traversals run in ONE persistent launch (replayed as a CUDA
  * graph).  Each block of the launch takes items from a device work counter
  * and runs an item's whole direction-optimizing level loop by itself, with
- * the item's own alpha, beta and degree threshold (warp_min, 32..256; 0 =
- * 32) -- the values the autotuner picks per graph-shape class.  No reference
+ * the item's own alpha and beta -- the values the autotuner picks per
+ * graph-shape class -- and, on graphs of more than 2^19 vertices, its degree
+ * threshold (warp_min, 32..256; 0 = 32).  The longest items are started
+ * first.  No reference
  * counterpart beyond one nw::graph::bfs call per item; results are the same.
  * Registration: graph g has graph_n[g] vertices; off_concat holds each
  * graph's n + 1 offsets (starting at 0) one graph after the other, col_concat
@@ -260,8 +266,8 @@ int nwg_ragged_release(nwg_ragged r);
 int nwg_ragged_info(nwg_ragged r, uint32_t* num_graphs, uint64_t* total_n, uint64_t* nmax, uint64_t* mmax);
 /* parents_dev: packed output, item i's parents (n of its graph) start at
  * item_offsets_host[i] (the running sum of the items' n, written when
- * non-NULL).  blocks_per_sm: resident blocks per SM of the persistent launch
- * (1..8, 0 = 2).  Synchronous; device_ms = device time of the launch. */
+ * non-NULL).  blocks_per_sm: most resident blocks per SM of the persistent
+ * launch (1..8, 0 = 2).  Synchronous; device_ms = device time of the launch. */
 int nwg_ragged_bfs(nwg_ragged r, uint32_t num_items, const nwg_ragged_item* items, uint32_t* parents_dev,
                    uint64_t* item_offsets_host, nwg_ragged_result* results_host, uint32_t blocks_per_sm,
                    float* device_ms);
@@ -335,11 +341,11 @@ int nwg_server_run_trace(nwg_server s, uint32_t count, const uint32_t* graph, co
  * GPU work overlaps race, so serialise them.  The first call on a device
  * looks the array's device address up and keeps it for the life of the
  * process: do not use this entry point on a device across cudaDeviceReset,
- * which unloads the module that holds the array.  The level loop is driven
- * from the host (a small read-back per step) on `stream` (a cudaStream_t,
- * NULL = legacy default stream) and the call synchronises that stream, so
- * it must not be called while the stream is being captured into a CUDA
- * graph; it returns when the traversal is complete. */
+ * which unloads the module that holds the array.  The traversal runs on
+ * `stream` (a cudaStream_t, NULL = legacy default stream) and the call
+ * synchronises that stream, so it must not be called while the stream is
+ * being captured into a CUDA graph; it returns when the traversal is
+ * complete. */
 int nwg_bfs_noalloc(const uint64_t* out_off, const uint32_t* out_col, const uint64_t* in_off, const uint32_t* in_col,
                     uint64_t n, uint32_t root, int alpha, int beta, uint32_t* parents_dev, void* stream);
 

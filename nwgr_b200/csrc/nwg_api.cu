@@ -105,6 +105,8 @@ void graph_free(GraphDev* g) {
   g->ms_workspaces.clear();
   g->default_ws = nullptr;
   g->pipe_ws    = nullptr;
+  roots_pool_free(g->roots_pool);
+  g->roots_pool = nullptr;
   if (g->owns_out) {
     cudaFree(g->off);
     cudaFree(g->col);
@@ -291,7 +293,8 @@ int bfs_sync(GraphDev* g, uint32_t root, int alpha, int beta, uint32_t* parents_
   return NWG_OK;
 }
 
-// k traversals with their parents copied to host rows, two in flight: the
+// k traversals with their parents copied to host rows.  On small graphs a
+// block per root (roots_run).  Otherwise two in flight: the
 // graph's default workspace and a second one take the roots in turn, each on
 // its own stream, so the device-to-host copy of root i's parents runs while
 // root i + 1 traverses (the traversals themselves run one after another:
@@ -308,6 +311,11 @@ int bfs_roots(GraphDev* g, const uint32_t* roots, uint64_t k, int alpha, int bet
   if (alpha <= 0 || beta <= 0) return set_error(NWG_EINVAL, "alpha and beta must be positive");
   std::lock_guard<std::mutex> lk(g->mu);
   DeviceGuard                 dg(g->device);
+  if (roots_by_block(g, k)) {
+    const int rb = roots_run(g, roots, k, alpha, beta, parents_host);
+    if (status) std::fill(status, status + k, (int32_t)rb);
+    return rb;
+  }
   Workspace*                  w[2] = {nullptr, nullptr};
   int                         rc   = get_default_ws(g, &w[0]);
   if (rc) return rc;

@@ -42,6 +42,7 @@
 // also carries such stale bits (curr is not cleared after bitmap->queue,
 // bfs.hpp:235-239).  Later pulls of the phase use the previous pull's C.
 #include <algorithm>
+#include <cmath>
 #include <cooperative_groups.h>
 
 #include "nwg_internal.cuh"
@@ -68,6 +69,17 @@ constexpr int kTdPerSm     = 4;   // k_td blocks per SM (64 registers per thread
 constexpr uint32_t kSoloCap    = 1024;
 constexpr uint32_t kSoloLevels = 256;
 constexpr uint32_t kSoloPer    = kSoloCap / kThreads;  // list entries per thread in the prefix pass
+// One-block traversals (nwg_block.cuh): threads of the block that runs a
+// single traversal and of the blocks that run many roots of a graph.
+constexpr int kBlkOneT   = 1024;
+constexpr int kBlkRootsT = 512;
+// A single traversal is one block's up to these sizes.  Device time of one
+// block against the whole grid (k_trav), B200: RMAT 2^10 21 / 64 us, 2^13
+// (204k edges) 32 / 72, uniform 2^13 (262k) 58 / 99, 2^14 (98k) 80 / 104,
+// grid 2^15 (131k) 330 / 412; past them the grid wins: uniform 2^14 (524k)
+// 118 / 64, 2^15 (197k) 130 / 115, grid 2^16 (262k) 548 / 458.
+constexpr uint64_t kBlkOneN = 1ull << 15;
+constexpr uint64_t kBlkOneM = 1ull << 18;
 
 __device__ __forceinline__ unsigned long long globaltimer() {
   unsigned long long t;
@@ -2085,9 +2097,76 @@ __global__ void k_widen(const uint32_t* __restrict__ src, uint64_t* __restrict__
     dst[i] = src[i];
 }
 
+#include "nwg_block.cuh"
+
+// One traversal by one block; leaves the control header as k_trav does.
+__global__ void __launch_bounds__(kBlkOneT)
+    k_blk_one(BlkGraph g, uint32_t root, uint32_t alpha, uint32_t beta, uint32_t topdown_only, uint32_t* parents,
+              BlkEnt* q, Ctrl* ctrl) {
+  extern __shared__ __align__(16) unsigned char blk_smem[];
+  uint32_t           ntr = 0;
+  const RaggedResult r =
+      block_traverse<kBlkOneT>(g, root, alpha, beta, topdown_only != 0, parents, q, blk_smem, ctrl, &ntr);
+  if (threadIdx.x == 0) {
+    CtrlHdr& c     = ctrl->h;
+    c.parents      = parents;
+    c.root         = root;
+    c.alpha        = alpha;
+    c.beta         = beta;
+    c.topdown_only = topdown_only;
+    c.action       = kActNone;
+    c.status       = r.status;
+    c.steps        = r.steps;
+    c.levels       = r.levels;
+    c.td_steps     = r.td_steps;
+    c.bu_steps     = r.bu_steps;
+    c.b2q_steps    = r.b2q_steps;
+    c.reached      = r.reached;
+    c.trace_len    = ntr;
+    ctrl->kernels  = 1;
+    ctrl->decides  = 0;
+    ctrl->err      = 0;
+  }
+}
+
+// A ragged batch's items [first, n_items), largest first: blocks take them
+// from a counter.  A queue of nmax entries per block in rp.scratch.
+template <int T>
+__global__ void __launch_bounds__(T, 1024 / T) k_blk_ragged(RaggedParams rp, uint32_t first, unsigned int* next) {
+  extern __shared__ __align__(16) unsigned char blk_smem[];
+  __shared__ uint32_t s_item;
+  BlkEnt* const       q = reinterpret_cast<BlkEnt*>(rp.scratch) + (uint64_t)blockIdx.x * rp.nmax;
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_item = first + atomicAdd(next, 1u);
+    __syncthreads();
+    const uint32_t it = s_item;
+    if (it >= rp.n_items) break;
+    const RaggedItem   item = rp.items[it];
+    const RaggedGraph  gr   = rp.graphs[item.graph];
+    const uint64_t*    off  = rp.off + gr.off_base;
+    const uint32_t*    col  = rp.col + gr.col_base;
+    const BlkGraph     g{off, col, off, col, rp.Z + gr.z_base, gr.n, gr.m};
+    const RaggedResult r = block_traverse<T>(g, item.root, (uint32_t)item.alpha, (uint32_t)item.beta, false,
+                                             rp.parents + item.out_base, q, blk_smem, nullptr, nullptr);
+    if (threadIdx.x == 0) rp.results[item.index] = r;
+  }
+}
+
+// Roots [0, k) of one graph, a block each (root i's parents in row i).
+__global__ void __launch_bounds__(kBlkRootsT, 1024 / kBlkRootsT)
+    k_blk_roots(BlkGraph g, const uint32_t* __restrict__ roots, uint32_t k, uint32_t alpha, uint32_t beta,
+                uint32_t* rows, BlkEnt* q) {
+  extern __shared__ __align__(16) unsigned char blk_smem[];
+  const uint32_t i = blockIdx.x;
+  if (i < k)
+    block_traverse<kBlkRootsT>(g, roots[i], alpha, beta, false, rows + i * g.n, q + i * g.n, blk_smem, nullptr,
+                               nullptr);
+}
+
 // ---------------------------------------------------------------------------
-// k_ragged: a ragged batch of (graph, root) traversals over many small packed
-// graphs in one persistent launch.  Each block takes items from an atomic
+// k_ragged: the items of a ragged batch whose graphs are too large for
+// k_blk_ragged (items [0, n_items) of the table).  Each block takes items from an atomic
 // counter and runs the whole level loop of one item by itself: the same
 // init / decide / top-down / bottom-up / bitmap->queue steps as the
 // single-graph path, with nblocks = 1 and __syncthreads() in place of
@@ -2178,7 +2257,7 @@ __global__ void __launch_bounds__(kThreads) k_ragged(RaggedParams rp) {
       r.bu_steps  = c.bu_steps;
       r.b2q_steps = c.b2q_steps;
       r.reached   = c.reached;
-      rp.results[it] = r;
+      rp.results[item.index] = r;
     }
     __syncthreads();
   }
@@ -2235,7 +2314,8 @@ int ws_init(GraphDev* g, Workspace* ws) {
   NWG_CUDA_TRY(cudaEventCreate(&ws->ev1));
   if (cudaMalloc(&ws->parents, std::max<uint64_t>(n, 4) * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&ws->V, 3ull * std::max<uint32_t>(nwords, 1) * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&ws->qbuf, 2ull * qs_cap * sizeof(uint32_t)) != cudaSuccess ||
+      cudaMalloc(&ws->qbuf, std::max<uint64_t>(2 * qs_cap * sizeof(uint32_t), blk_one_fits(n, m) ? n * sizeof(BlkEnt) : 0)) !=
+          cudaSuccess ||
       cudaMalloc(&ws->cbuf, 2ull * qc_cap * sizeof(uint64_t)) != cudaSuccess ||
       cudaMalloc(&ws->hubbuf, 2ull * hub_cap * sizeof(HubRec)) != cudaSuccess ||
       cudaMalloc(&ws->ctrl, sizeof(Ctrl)) != cudaSuccess) {
@@ -2339,8 +2419,51 @@ static int coop_launch(const void* fn, dim3 grid, void** args, cudaStream_t stre
   return NWG_OK;
 }
 
-// A traversal on `stream`: the persistent traversal kernel, one cooperative
-// launch after clearing its barrier's arrival count.
+// A block's time over one item grows with the vertices and, as few edges per
+// vertex mean many levels and long top-down phases, more per vertex on sparse
+// graphs: measured 8.0 (grid), 4.0 (degree 6), 2.4 ns a vertex (degree 32)
+// at 2^16-2^18 vertices.
+double blk_weight(uint64_t n, uint64_t m) { return (double)n * (1.0 + 8.0 * (double)n / (double)std::max<uint64_t>(m, 1)); }
+
+// Raises a kernel's dynamic shared memory limit to what a block may have,
+// once per device.
+template <auto kernel>
+static int blk_prepare() {
+  static std::mutex        mu;
+  static std::vector<char> done;  // per device
+  int                      dev = 0;
+  NWG_CUDA_TRY(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  if ((int)done.size() <= dev) done.resize(dev + 1, 0);
+  if (!done[dev]) {
+    cudaFuncAttributes fa;
+    NWG_CUDA_TRY(cudaFuncGetAttributes(&fa, (const void*)kernel));
+    int optin = 0;
+    NWG_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    NWG_CUDA_TRY(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      optin - (int)fa.sharedSizeBytes));
+    done[dev] = 1;
+  }
+  return NWG_OK;
+}
+
+static BlkGraph blk_graph(const DobfsParams& P) { return BlkGraph{P.off, P.col, P.in_off, P.in_col, P.Z, P.n, P.m}; }
+
+bool blk_one_fits(uint64_t n, uint64_t m) { return n <= kBlkOneN && m <= kBlkOneM; }
+
+static int blk_one_launch(const BlkGraph& g, uint32_t root, int alpha, int beta, uint32_t* parents, BlkEnt* q,
+                          Ctrl* ctrl, bool topdown_only, cudaStream_t stream) {
+  const int rc = blk_prepare<k_blk_one>();
+  if (rc) return rc;
+  k_blk_one<<<1, kBlkOneT, blk_smem_bytes<kBlkOneT>(g.n), stream>>>(g, root, (uint32_t)alpha, (uint32_t)beta,
+                                                                    topdown_only ? 1u : 0u, parents, q, ctrl);
+  NWG_CUDA_TRY(cudaGetLastError());
+  return NWG_OK;
+}
+
+// A traversal on `stream`: one block for a small graph, else the persistent
+// traversal kernel, one cooperative launch after clearing its barrier's
+// arrival count.
 int ws_launch(Workspace* ws, uint32_t root, int alpha, int beta, uint32_t* parents, cudaStream_t stream,
               bool topdown_only) {
   GraphDev* g = ws->g;
@@ -2348,11 +2471,127 @@ int ws_launch(Workspace* ws, uint32_t root, int alpha, int beta, uint32_t* paren
   if (alpha <= 0 || beta <= 0) return set_error(NWG_EINVAL, "alpha and beta must be positive");
   uint32_t  r = root, a = (uint32_t)alpha, b = (uint32_t)beta, td = topdown_only ? 1u : 0u;
   uint32_t* par    = parents ? parents : ws->parents;
+  if (blk_one_fits(g->n, g->m)) {
+    const int rc = blk_one_launch(blk_graph(ws->params), root, alpha, beta, par,
+                                  reinterpret_cast<BlkEnt*>(ws->qbuf), ws->ctrl, topdown_only, stream);
+    if (rc) return rc;
+    ws->ran = true;
+    return NWG_OK;
+  }
   void*     args[] = {&ws->params, &r, &a, &b, &par, &td};
   NWG_CUDA_TRY(cudaMemsetAsync(&ws->ctrl->bar, 0, sizeof(GridBar), stream));
   const int rc = coop_launch((const void*)k_trav, dim3(ws->trav_grid), args, stream);
   if (rc) return rc;
   ws->ran = true;
+  return NWG_OK;
+}
+
+// The same on state the caller owns (params without a workspace): q has room
+// for the graph's vertices where blk_one_fits.  Allocates no device memory.
+int run_traversal(const DobfsParams& params, int sm_count, uint32_t root, int alpha, int beta, uint32_t* parents,
+                  void* q, cudaStream_t stream) {
+  DobfsParams P = params;
+  if (blk_one_fits(P.n, P.m)) {
+    BlkGraph g = blk_graph(P);
+    g.Z        = nullptr;  // not built
+    return blk_one_launch(g, root, alpha, beta, parents, static_cast<BlkEnt*>(q), P.ctrl, false, stream);
+  }
+  const int rc = zero_indegree_into(P.in_off, P.n, const_cast<uint32_t*>(P.Z), sm_count, stream);
+  if (rc) return rc;
+  uint32_t r = root, a = (uint32_t)alpha, b = (uint32_t)beta, td = 0u;
+  void*    args[] = {&P, &r, &a, &b, &parents, &td};
+  NWG_CUDA_TRY(cudaMemsetAsync(&P.ctrl->bar, 0, sizeof(GridBar), stream));
+  return coop_launch((const void*)k_trav, dim3(resident_grid(sm_count, k_trav, kTravPerSm)), args, stream);
+}
+
+// Many roots of one graph, a block each.  A chunk of roots is one launch and
+// one copy of its rows; two chunks are in flight, each with its own rows,
+// queues and stream, so a chunk's rows cross to the host while the next
+// traverses.
+struct RootsPool {
+  struct Lane {
+    uint32_t     slots = 0;  // roots its buffers hold
+    uint32_t*    roots = nullptr;
+    uint32_t*    rows  = nullptr;
+    BlkEnt*      q     = nullptr;
+    cudaStream_t s     = nullptr;
+  } lane[2];
+};
+
+static void lane_free(RootsPool::Lane& l) {
+  if (l.s) {
+    cudaStreamSynchronize(l.s);
+    cudaStreamDestroy(l.s);
+  }
+  cudaFree(l.roots);
+  cudaFree(l.rows);
+  cudaFree(l.q);
+  l = RootsPool::Lane{};
+}
+
+void roots_pool_free(RootsPool* p) {
+  if (!p) return;
+  for (auto& l : p->lane) lane_free(l);
+  delete p;
+}
+
+constexpr uint64_t kRootsPoolBytes = 128ull << 20;  // rows and queues of the two chunks
+
+// Blocks two to an SM, fewer where the pool's memory bound says so.
+static uint32_t roots_slots(const GraphDev* g) {
+  const uint64_t per = 2 * std::max<uint64_t>(g->n, 1) * (sizeof(uint32_t) + sizeof(BlkEnt));
+  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(2ull * g->sm_count, kRootsPoolBytes / per));
+}
+
+// A block takes about 20 us and 4 ns per weighted vertex (kBlkRootsT
+// threads) for a root, side by side with the launch's others; the grid 60 us
+// or more for each root, one after another (its traversals of graphs of up
+// to 2^19 vertices: 61-590 us).
+bool roots_by_block(const GraphDev* g, uint64_t k) {
+  if (g->n > kBlkMaxN || g->m >= kBlkMaxM || k < 2) return false;
+  const double waves = std::ceil((double)k / roots_slots(g));
+  return waves * (20.0 + 0.004 * blk_weight(g->n, g->m)) < 60.0 * (double)k;
+}
+
+int roots_run(GraphDev* g, const uint32_t* roots, uint64_t k, int alpha, int beta, uint32_t* parents_host) {
+  const uint64_t n  = g->n;
+  const int      rc = blk_prepare<k_blk_roots>();
+  if (rc) return rc;
+  const uint32_t chunk = (uint32_t)std::min<uint64_t>(k, roots_slots(g));
+  if (!g->roots_pool) g->roots_pool = new RootsPool();
+  for (int j = 0; j < (k > chunk ? 2 : 1); ++j) {
+    RootsPool::Lane& l = g->roots_pool->lane[j];
+    if (l.slots >= chunk) continue;
+    lane_free(l);
+    if (cudaMalloc(&l.roots, chunk * sizeof(uint32_t)) != cudaSuccess ||
+        cudaMalloc(&l.rows, chunk * n * sizeof(uint32_t)) != cudaSuccess ||
+        cudaMalloc(&l.q, chunk * (n <= kBlkSmemQ ? 1 : n) * sizeof(BlkEnt)) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&l.s, cudaStreamNonBlocking) != cudaSuccess) {
+      cudaGetLastError();
+      lane_free(l);
+      return set_error(NWG_ENOMEM, "buffers of a traversal over many roots (n=" + std::to_string(n) + ")");
+    }
+    l.slots = chunk;
+  }
+  const BlkGraph bg{g->off, g->col, g->in_off, g->in_col, g->Z, g->n, g->m};
+  cudaError_t    e = cudaSuccess;
+  for (uint64_t i = 0; i < k && e == cudaSuccess; i += chunk) {
+    const RootsPool::Lane& l = g->roots_pool->lane[(i / chunk) & 1];
+    const uint32_t         c = (uint32_t)std::min<uint64_t>(chunk, k - i);
+    e = cudaMemcpyAsync(l.roots, roots + i, c * sizeof(uint32_t), cudaMemcpyHostToDevice, l.s);
+    if (e != cudaSuccess) break;
+    k_blk_roots<<<c, kBlkRootsT, blk_smem_bytes<kBlkRootsT>(n), l.s>>>(bg, l.roots, c, (uint32_t)alpha, (uint32_t)beta,
+                                                                       l.rows, l.q);
+    e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(parents_host + i * n, l.rows, c * n * sizeof(uint32_t), cudaMemcpyDeviceToHost, l.s);
+  }
+  for (const auto& l : g->roots_pool->lane) {
+    if (!l.s) continue;
+    const cudaError_t w = cudaStreamSynchronize(l.s);
+    if (e == cudaSuccess) e = w;
+  }
+  if (e != cudaSuccess) return cuda_error(e, "traversals over many roots");
   return NWG_OK;
 }
 
@@ -2522,11 +2761,6 @@ int depth_row16(Workspace* ws, uint32_t root, uint16_t* row, cudaStream_t stream
   return NWG_OK;
 }
 
-int ragged_slot_bytes(uint64_t nmax, uint64_t mmax, uint64_t* bytes) {
-  *bytes = slot_layout(nmax, mmax).bytes;
-  return NWG_OK;
-}
-
 int zero_indegree_packed(RaggedDev* r) {
   if (r->ngraphs == 0) return NWG_OK;
   k_zero_indegree_packed<<<std::max(1, r->sm_count * 4), kThreads>>>(r->off, r->graphs, r->ngraphs, r->Z);
@@ -2534,12 +2768,71 @@ int zero_indegree_packed(RaggedDev* r) {
   return NWG_OK;
 }
 
-// One persistent launch over the r->items table (already on the device),
-// captured into a CUDA graph with the counter reset and replayed while the
-// item count, slot count and output buffer stay the same.
-int ragged_launch(RaggedDev* r, uint32_t n_items, uint32_t* parents_dev, uint32_t blocks_per_sm, float* ms) {
-  const uint32_t slots = (uint32_t)std::max(1, r->sm_count * (int)blocks_per_sm);
-  if (!r->exec || r->exec_items != n_items || r->exec_slots != slots || r->exec_parents != parents_dev) {
+// Items [0, n_big) by k_ragged, the others by k_blk_ragged, into the
+// capturing stream.
+template <int T>
+static int blk_ragged_enqueue(RaggedDev* r, const RaggedParams& rp, uint32_t n_big, uint32_t slots) {
+  const int rc = blk_prepare<k_blk_ragged<T>>();
+  if (rc) return rc;
+  k_blk_ragged<T><<<slots, T, blk_smem_bytes_upto<T>(r->blk_nmax), r->stream>>>(rp, n_big, rp.next_item + 1);
+  NWG_CUDA_TRY(cudaGetLastError());
+  return NWG_OK;
+}
+
+// Whether an item of a graph of n vertices and m entries is one block's
+// (k_blk_ragged) or k_ragged's.
+bool ragged_by_block(uint64_t n, uint64_t m) { return n <= kBlkMaxN && m < kBlkMaxM; }
+
+// Threads per block of k_blk_ragged.  Two blocks of 512 per SM finish more
+// items in all (items of 2^10..2^14 vertices: 0.33 against 0.48 ms), one of
+// 1,024 finishes a large item sooner (2^10..2^18 vertices, where the largest
+// grid alone takes 2 ms: 2.2 against 4.4 ms).  A 512-thread block takes about
+// 1.65 times as long for an item, so 512 where even so the largest item ends
+// before the others' work does.
+int ragged_block_threads(const RaggedDev* r, double max_weight, double sum_weight, uint32_t blocks_per_sm) {
+  const bool two = blocks_per_sm >= 2 && 2 * (blk_smem_bytes_upto<512>(r->blk_nmax) + 1024) <= 227 * 1024;
+  return two && 1.65 * max_weight * r->sm_count < sum_weight ? 512 : 1024;
+}
+
+// Blocks of the launch that are resident at once (a block takes items until
+// none is left, so more would find none), and the scratch of a launch: a
+// slot per k_ragged block, or a queue per k_blk_ragged block.
+static uint32_t ragged_slots(const RaggedDev* r, uint32_t blocks_per_sm, int threads) {
+  return (uint32_t)std::max(1, r->sm_count * (int)std::min(blocks_per_sm, 1024u / (uint32_t)threads));
+}
+uint64_t ragged_scratch_bytes(const RaggedDev* r, bool any_big, uint32_t blocks_per_sm, int threads) {
+  const uint64_t queues = ragged_slots(r, blocks_per_sm, threads) * std::max<uint64_t>(r->blk_nmax, 1) * sizeof(BlkEnt);
+  if (!any_big) return queues;
+  return std::max<uint64_t>(queues, (uint64_t)r->sm_count * blocks_per_sm * slot_layout(r->nmax, r->mmax).bytes);
+}
+
+static int ragged_enqueue(RaggedDev* r, const RaggedParams& rp, uint32_t n_big, uint32_t blocks_per_sm, int threads) {
+  NWG_CUDA_TRY(cudaMemsetAsync(r->counter, 0, 2 * sizeof(unsigned int), r->stream));
+  if (n_big) {
+    RaggedParams big = rp;
+    big.n_items      = n_big;
+    k_ragged<<<r->sm_count * blocks_per_sm, kThreads, 0, r->stream>>>(big);
+    NWG_CUDA_TRY(cudaGetLastError());
+  }
+  if (n_big < rp.n_items) {
+    RaggedParams small = rp;
+    small.nmax         = r->blk_nmax;
+    const uint32_t slots = ragged_slots(r, blocks_per_sm, threads);
+    const int      rc    = threads == 512 ? blk_ragged_enqueue<512>(r, small, n_big, slots)
+                                          : blk_ragged_enqueue<1024>(r, small, n_big, slots);
+    if (rc) return rc;
+  }
+  return NWG_OK;
+}
+
+// The r->items table (already on the device; its first n_big items are
+// k_ragged's), captured into a CUDA graph with the counters' reset and
+// replayed while the item counts, blocks per SM, block size and output
+// buffer stay the same.
+int ragged_launch(RaggedDev* r, uint32_t n_items, uint32_t n_big, uint32_t* parents_dev, uint32_t blocks_per_sm,
+                  int threads, float* ms) {
+  if (!r->exec || r->exec_items != n_items || r->exec_big != n_big || r->exec_per_sm != blocks_per_sm ||
+      r->exec_threads != threads || r->exec_parents != parents_dev) {
     if (r->exec) {
       cudaGraphExecDestroy(r->exec);
       r->exec = nullptr;
@@ -2560,17 +2853,21 @@ int ragged_launch(RaggedDev* r, uint32_t n_items, uint32_t* parents_dev, uint32_
     rp.mmax         = r->mmax;
     cudaGraph_t graph;
     NWG_CUDA_TRY(cudaStreamBeginCapture(r->stream, cudaStreamCaptureModeThreadLocal));
-    cudaMemsetAsync(r->counter, 0, sizeof(unsigned int), r->stream);
-    k_ragged<<<slots, kThreads, 0, r->stream>>>(rp);
-    const cudaError_t le = cudaGetLastError();
+    const int         rc = ragged_enqueue(r, rp, n_big, blocks_per_sm, threads);
     const cudaError_t ce = cudaStreamEndCapture(r->stream, &graph);
-    if (le != cudaSuccess) return cuda_error(le, "k_ragged launch (capture)");
+    if (rc) {
+      if (ce == cudaSuccess) cudaGraphDestroy(graph);
+      cudaGetLastError();
+      return rc;
+    }
     if (ce != cudaSuccess) return cuda_error(ce, "cudaStreamEndCapture(ragged)");
     const cudaError_t ie = cudaGraphInstantiate(&r->exec, graph, 0);
     cudaGraphDestroy(graph);
     if (ie != cudaSuccess) return cuda_error(ie, "cudaGraphInstantiate(ragged)");
     r->exec_items   = n_items;
-    r->exec_slots   = slots;
+    r->exec_big     = n_big;
+    r->exec_per_sm  = blocks_per_sm;
+    r->exec_threads = threads;
     r->exec_parents = parents_dev;
   }
   NWG_CUDA_TRY(cudaEventRecord(r->ev0, r->stream));

@@ -225,8 +225,8 @@ struct RaggedItem {  // one (graph, root) traversal
   uint64_t out_base;  // index of the item's parents in the packed output
   int32_t  alpha;
   int32_t  beta;
-  uint32_t warp_min;  // degree threshold of the chunked queue
-  uint32_t pad;
+  uint32_t warp_min;  // degree threshold of the chunked queue (k_ragged)
+  uint32_t index;     // the item's place in the caller's table (its result's)
 };
 
 struct RaggedResult {
@@ -245,7 +245,7 @@ struct RaggedParams {
   uint32_t*           parents;
   uint32_t            n_items;
   unsigned int*       next_item;
-  unsigned char*      scratch;  // one slot per resident block
+  unsigned char*      scratch;  // one slot (k_ragged) or queue (k_blk_ragged) per resident block
   uint64_t            slot_bytes;
   uint64_t            nmax, mmax;
 };
@@ -255,6 +255,7 @@ struct RaggedDev {
   int                      sm_count = 148;
   uint32_t                 ngraphs  = 0;
   uint64_t                 nmax = 0, mmax = 0, total_n = 0;
+  uint64_t                 blk_nmax = 0;  // most vertices of a graph whose items are one block's
   uint64_t*                off      = nullptr;
   uint32_t*                col      = nullptr;
   uint32_t*                Z        = nullptr;
@@ -269,7 +270,8 @@ struct RaggedDev {
   cudaStream_t             stream   = nullptr;
   cudaEvent_t              ev0 = nullptr, ev1 = nullptr;
   cudaGraphExec_t          exec     = nullptr;
-  uint32_t                 exec_items = 0, exec_slots = 0;
+  uint32_t                 exec_items = 0, exec_big = 0, exec_per_sm = 0;
+  int                      exec_threads = 0;
   uint32_t*                exec_parents = nullptr;
   std::mutex               mu;
 };
@@ -292,6 +294,7 @@ struct GraphDev {
   std::mutex                mu;
   Workspace*                default_ws = nullptr;
   Workspace*                pipe_ws    = nullptr;  // second lane of nwg_bfs_roots
+  struct RootsPool*         roots_pool = nullptr;  // its rows and queues where blocks take the roots
   std::vector<Workspace*>   workspaces;
   std::vector<MsWorkspace*> ms_workspaces;
 };
@@ -322,8 +325,18 @@ int  build_deg16(GraphDev* g, cudaStream_t stream);
 int  component_edges(GraphDev* g, const uint32_t* parents, uint64_t* edges, uint64_t* vertices);
 int  widen_offsets(const uint32_t* src, uint64_t* dst, uint64_t count, cudaStream_t stream);
 
-int  ragged_launch(RaggedDev* r, uint32_t n_items, uint32_t* parents_dev, uint32_t blocks_per_sm, float* ms);
-int  ragged_slot_bytes(uint64_t nmax, uint64_t mmax, uint64_t* bytes);
+int  ragged_launch(RaggedDev* r, uint32_t n_items, uint32_t n_big, uint32_t* parents_dev, uint32_t blocks_per_sm,
+                   int threads, float* ms);
+int    ragged_block_threads(const RaggedDev* r, double max_weight, double sum_weight, uint32_t blocks_per_sm);
+double blk_weight(uint64_t n, uint64_t m);
+uint64_t ragged_scratch_bytes(const RaggedDev* r, bool any_big, uint32_t blocks_per_sm, int threads);
+bool ragged_by_block(uint64_t n, uint64_t m);
+bool blk_one_fits(uint64_t n, uint64_t m);
+bool roots_by_block(const GraphDev* g, uint64_t k);
+int  roots_run(GraphDev* g, const uint32_t* roots, uint64_t k, int alpha, int beta, uint32_t* parents_host);
+void roots_pool_free(struct RootsPool* p);
+int  run_traversal(const DobfsParams& params, int sm_count, uint32_t root, int alpha, int beta, uint32_t* parents,
+                   void* q, cudaStream_t stream);
 int  zero_indegree_packed(RaggedDev* r);
 
 // nwg_msbfs.cu

