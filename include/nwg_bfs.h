@@ -391,7 +391,8 @@ int nwg_graph_write_nwbin(nwg_graph g, const char* path);
 /* Device BFSVerifier: the checks of nw::graph::BFSVerifier(g, g_t, source,
  * parent) (reference: include/nwgraph/algorithms/bfs.hpp:44-98) on the GPU,
  * for a parent array in host OR device memory (exactly one non-NULL).  Depths
- * come from a plain top-down BFS written only for this check.  valid = 1 when
+ * come from a BFS written only for this check.  Its state (about 20 n + m / 32
+ * bytes) is kept with the graph; calls on one graph take turns.  valid = 1 when
  * the reference verifier would return true; otherwise first_bad is the
  * lowest failing vertex (the one the reference stops at) and reason the
  * reference's failure: 1 source wrong, 2 wrong depths, 3 no edge from the

@@ -107,6 +107,8 @@ void graph_free(GraphDev* g) {
   g->pipe_ws    = nullptr;
   roots_pool_free(g->roots_pool);
   g->roots_pool = nullptr;
+  verify_ws_free(g->verify_ws);
+  g->verify_ws = nullptr;
   if (g->owns_out) {
     cudaFree(g->off);
     cudaFree(g->col);

@@ -294,6 +294,7 @@ struct GraphDev {
   std::mutex                mu;
   Workspace*                default_ws = nullptr;
   Workspace*                pipe_ws    = nullptr;  // second lane of nwg_bfs_roots
+  struct VerifyWs*          verify_ws  = nullptr;  // state of nwg_verify
   struct RootsPool*         roots_pool = nullptr;  // its rows and queues where blocks take the roots
   std::vector<Workspace*>   workspaces;
   std::vector<MsWorkspace*> ms_workspaces;
@@ -338,6 +339,9 @@ void roots_pool_free(struct RootsPool* p);
 int  run_traversal(const DobfsParams& params, int sm_count, uint32_t root, int alpha, int beta, uint32_t* parents,
                    void* q, cudaStream_t stream);
 int  zero_indegree_packed(RaggedDev* r);
+
+// nwg_verify.cu
+void verify_ws_free(struct VerifyWs* b);
 
 // nwg_msbfs.cu
 int      ms_ws_init(GraphDev* g, MsWorkspace* ws);

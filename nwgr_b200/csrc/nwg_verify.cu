@@ -2,9 +2,9 @@
 // parent) (include/nwgraph/algorithms/bfs.hpp:44-98 in NWGraph) on the GPU.
 //
 //   1. depth = BFS depths from the source over the out-graph (bfs.hpp:47-63).
-//      Computed by a plain level-synchronous top-down BFS written only for
-//      this check (a warp per frontier vertex, atomicCAS on depth): it shares
-//      no code with the direction-optimizing kernels it is used to verify.
+//      Computed by a plain level-synchronous BFS written only for this check:
+//      it shares no code with the direction-optimizing kernels it is used to
+//      verify.
 //   2. For every vertex u (bfs.hpp:64-96): when depth[u] and parent[u] are
 //      both set, the source must be its own parent at depth 0, and any other
 //      u must find parent[u] among its in-neighbours (g_t) with
@@ -15,7 +15,23 @@
 // every vertex is checked in parallel and the lowest failing one is kept
 // (a 64-bit atomicMin on vertex << 3 | reason), so the verdict, the vertex
 // and the reason are the ones the reference reports.
+//
+// The depths' BFS: a level either pushes from a queue of 64-edge pieces of
+// its vertices (so a hub is spread over the grid: with a warp per vertex the
+// hub level of RMAT-22 alone took 4.6 of 10.4 ms) or, when its out-edges are
+// many, pulls over the visited bitmap.  No unvisited vertex has an
+// in-neighbour of an earlier level than the last complete one (that level
+// would have visited it), so every visited in-neighbour is one level up; the
+// pull reads one copy of the bitmap and writes the other, whose difference
+// afterwards is the level.  A level is two launches that read the level's
+// counts from device memory (building the queue after a pull; the step), so
+// the host enqueues many levels and reads the counts back once.
+//
+// Bound: gathers of single visited bits and columns (latency); RMAT-22 on a
+// B200: 0.5 ms against 10.4 with a warp per frontier vertex and a lane's
+// in-edges tested one by one.
 #include <algorithm>
+#include <mutex>
 #include <string>
 
 #include "nwg_internal.cuh"
@@ -28,74 +44,275 @@ namespace {
 
 constexpr int      kVThreads = 256;
 constexpr uint32_t kUnset    = 0xFFFFFFFFu;  // std::numeric_limits<uint32_t>::max()
+constexpr uint32_t kVPiece   = 64;           // out-edges per queue entry: eight lanes, eight edges each
+constexpr uint32_t kVProbe   = 8;            // in-edges a lane reads per round
+constexpr uint32_t kVLane    = 32;           // in-edges a lane scans alone before the warp helps
+constexpr uint32_t kVHub     = 1024;         // a longer rest of a list is checked by the grid, in pieces of this
+constexpr uint32_t kVBatch   = 32;           // most levels enqueued before the counts are read back
 
-struct VerifyCounters {
-  unsigned long long next;     // vertices appended to the next frontier
-  unsigned long long first;    // min over failing vertices of (u << 3 | reason)
-  unsigned long long reached;  // vertices with a depth
+// One level's frontier, complete when its step runs.
+struct VerifyLevel {
+  unsigned long long verts;      // vertices of the level
+  unsigned long long edges;      // their out-edges
+  unsigned long long entries;    // queue entries
+  unsigned long long unpushed;   // out-edges of the graph not yet of any level before
+  unsigned int       from_pull;  // found by a pull: the queue is not built
+  unsigned int       cur;        // which copy of the visited bitmap is current
 };
 
-__global__ void k_v_init(uint32_t* depth, uint64_t n, uint32_t source, uint32_t* q0, VerifyCounters* cnt) {
+struct VerifyCounters {
+  unsigned long long first;    // min over failing vertices of (u << 3 | reason)
+  unsigned long long reached;  // vertices with a depth
+  unsigned long long pieces;   // pieces of long in-lists
+  unsigned long long pad;
+  VerifyLevel        lv[kVBatch + 1];
+};
+
+struct VerifyArgs {
+  const uint64_t* off;
+  const uint32_t* col;
+  const uint64_t* in_off;
+  const uint32_t* in_col;
+  uint64_t        n, m;
+  uint32_t*       depth;
+  uint32_t*       vis[2];  // visited bitmap, two copies
+  uint64_t*       q[2];    // vertex << 32 | piece
+  uint64_t        qcap;
+  VerifyCounters* cnt;
+};
+
+// Pull when the level's out-edges are a good part of what is left (and not
+// a handful), or its queue entries did not fit (more than n + m / 512
+// entries: over m / 8 out-edges).
+__device__ __forceinline__ bool v_pulls(const VerifyArgs& a, const VerifyLevel& l) {
+  return l.entries > a.qcap || (l.edges > l.unpushed / 15 && l.edges > a.n / 32);
+}
+
+__global__ void k_v_init(VerifyArgs a, uint32_t source) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-    depth[i] = (i == source) ? 0u : kUnset;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    q0[0]        = source;
-    cnt->next    = 0;
-    cnt->first   = ~0ull;
-    cnt->reached = 0;
+  const uint64_t t      = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t deg    = a.off[source + 1] - a.off[source];
+  const uint64_t np     = (deg + kVPiece - 1) / kVPiece;
+  for (uint64_t i = t; i < a.n; i += stride) a.depth[i] = (i == source) ? 0u : kUnset;
+  for (uint64_t w = t; w < (a.n + 31) / 32; w += stride)
+    a.vis[0][w] = w == source >> 5 ? 1u << (source & 31) : 0u;
+  for (uint64_t i = t; i < np && i < a.qcap; i += stride) a.q[0][i] = ((uint64_t)source << 32) | i;
+  if (t == 0) {
+    a.cnt->first   = ~0ull;
+    a.cnt->reached = 0;
+    a.cnt->pieces  = 0;
+    a.cnt->lv[0]   = VerifyLevel{1, deg, np, a.m, 0, 0};
   }
 }
 
-// One level: every out-edge of the frontier claims unvisited targets.
-__global__ void __launch_bounds__(kVThreads) k_v_level(const uint64_t* __restrict__ off,
-                                                       const uint32_t* __restrict__ col, uint32_t* depth,
-                                                       const uint32_t* __restrict__ q, uint64_t qsize, uint32_t* qn,
-                                                       uint64_t qcap, uint32_t level, VerifyCounters* cnt) {
-  const unsigned lane   = threadIdx.x & 31;
-  const uint64_t gwarp  = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t i = gwarp; i < qsize; i += nwarps) {
-    const uint32_t u   = q[i];
-    const uint64_t beg = off[u], end = off[u + 1];
-    for (uint64_t e0 = beg; e0 < end; e0 += 32) {
-      const uint64_t e   = e0 + lane;
-      bool           won = false;
-      uint32_t       v   = 0;
-      if (e < end) {
-        v   = col[e];
-        won = depth[v] == kUnset && atomicCAS(&depth[v], kUnset, level + 1) == kUnset;
+// Appends the warp's vertices (lane's v where `has`, out-degree deg) to q as
+// pieces.  All lanes call.
+__device__ __forceinline__ void v_append(const VerifyArgs& a, uint64_t* q, unsigned long long* entries, bool has,
+                                         uint32_t v, uint64_t deg) {
+  const unsigned     lane = threadIdx.x & 31;
+  const uint64_t     np   = has ? (deg + kVPiece - 1) / kVPiece : 0;
+  unsigned long long inc  = np;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long x = __shfl_up_sync(kFullMask, inc, o);
+    if ((int)lane >= o) inc += x;
+  }
+  const unsigned long long tot = __shfl_sync(kFullMask, inc, 31);
+  if (tot == 0) return;
+  unsigned long long base = 0;
+  if (lane == 31) base = atomicAdd(entries, tot);
+  base                         = __shfl_sync(kFullMask, base, 31);
+  const unsigned long long pos = base + inc - np;
+  if (np && np <= 8)
+    for (uint64_t j = 0; j < np; ++j)
+      if (pos + j < a.qcap) q[pos + j] = ((uint64_t)v << 32) | j;
+  unsigned big = __ballot_sync(kFullMask, np > 8);
+  while (big) {  // the whole warp writes a hub's
+    const int src = __ffs(big) - 1;
+    big &= big - 1;
+    const uint64_t           vs = __shfl_sync(kFullMask, (uint64_t)v, src);
+    const unsigned long long ps = __shfl_sync(kFullMask, pos, src);
+    const uint64_t           ns = __shfl_sync(kFullMask, np, src);
+    for (uint64_t j = lane; j < ns; j += 32)
+      if (ps + j < a.qcap) q[ps + j] = (vs << 32) | j;
+  }
+}
+
+// The queue of level L, when it was found by a pull and will push.
+__global__ void __launch_bounds__(kVThreads) k_v_queue(VerifyArgs a, uint32_t L, uint32_t q) {
+  VerifyLevel& l = a.cnt->lv[L];
+  if (l.verts == 0 || !l.from_pull || v_pulls(a, VerifyLevel{l.verts, l.edges, 0, l.unpushed, 0, 0})) return;
+  const uint32_t* cur    = a.vis[l.cur];
+  const uint32_t* old    = a.vis[l.cur ^ 1];
+  const unsigned  lane   = threadIdx.x & 31;
+  const uint64_t  nwords = (a.n + 31) / 32;
+  const uint64_t  nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nwords; w += nwarps) {
+    const uint32_t d = cur[w] ^ old[w];
+    if (!d) continue;
+    const bool     has = (d >> lane) & 1u;
+    const uint32_t v   = (uint32_t)(w * 32 + lane);
+    v_append(a, a.q[q], &l.entries, has, v, has ? a.off[v + 1] - a.off[v] : 0);
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ T v_block_sum(T x) {
+  __shared__ T red[kVThreads / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(kFullMask, x, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
+  __syncthreads();
+  T t = 0;
+#pragma unroll
+  for (int i = 0; i < kVThreads / 32; ++i) t += red[i];
+  return t;
+}
+
+// The step of level L (depth `level`): discoveries get depth level + 1 and
+// are counted in lv[L + 1].
+__global__ void __launch_bounds__(kVThreads) k_v_step(VerifyArgs a, uint32_t L, uint32_t q, uint32_t level) {
+  const VerifyLevel l  = a.cnt->lv[L];
+  VerifyLevel&      nl = a.cnt->lv[L + 1];
+  if (l.verts == 0) return;
+  const bool         pull  = v_pulls(a, l);
+  const unsigned     lane  = threadIdx.x & 31;
+  const uint64_t     warp  = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint64_t     nwarp = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  unsigned long long verts = 0, edges = 0;
+  uint32_t* const    cur   = a.vis[l.cur];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    nl.unpushed  = l.unpushed - min(l.unpushed, l.edges);
+    nl.from_pull = pull;
+    nl.cur       = l.cur ^ (pull ? 1u : 0u);
+  }
+  if (pull) {
+    uint32_t* const next   = a.vis[l.cur ^ 1];
+    const uint64_t  nwords = (a.n + 31) / 32;
+    for (uint64_t w = warp; w < nwords; w += nwarp) {
+      const uint32_t seen = cur[w];
+      const uint32_t u    = (uint32_t)(w * 32 + lane);
+      bool           need = u < a.n && !((seen >> lane) & 1u);
+      uint64_t       e = 0, end = 0;
+      if (need) {
+        e    = a.in_off[u];
+        end  = a.in_off[u + 1];
+        need = e < end;
       }
-      const unsigned m = __ballot_sync(kFullMask, won);
-      if (m) {
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(&cnt->next, (unsigned long long)__popc(m));
-        base = __shfl_sync(kFullMask, base, 0);
-        if (won) {
-          const uint64_t at = base + __popc(m & ((1u << lane) - 1u));
-          if (at < qcap) qn[at] = v;
+      bool           found = false;
+      const uint64_t lim   = min(end, e + kVLane);
+      while (need && e < lim) {
+        uint32_t x[kVProbe];
+#pragma unroll
+        for (uint32_t k = 0; k < kVProbe; ++k) x[k] = e + k < lim ? __ldg(a.in_col + e + k) : kUnset;
+#pragma unroll
+        for (uint32_t k = 0; k < kVProbe; ++k)
+          if (x[k] != kUnset && ((cur[x[k] >> 5] >> (x[k] & 31)) & 1u)) found = true;
+        e += kVProbe;
+        if (found) need = false;
+      }
+      unsigned pend = __ballot_sync(kFullMask, need && e < end);
+      while (pend) {  // the rest of long lists: the warp together
+        const int ld = __ffs(pend) - 1;
+        pend &= pend - 1;
+        const uint64_t b  = __shfl_sync(kFullMask, e, ld);
+        const uint64_t en = __shfl_sync(kFullMask, end, ld);
+        bool           hit = false;
+        for (uint64_t base = b; base < en && !hit; base += 32 * 4) {
+          uint32_t x[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) x[k] = base + k * 32 + lane < en ? __ldg(a.in_col + base + k * 32 + lane) : kUnset;
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (x[k] != kUnset && ((cur[x[k] >> 5] >> (x[k] & 31)) & 1u)) hit = true;
+          hit = __any_sync(kFullMask, hit);
         }
+        if ((int)lane == ld) found = hit;
+      }
+      const uint32_t fresh = __ballot_sync(kFullMask, found);
+      if (found) {
+        a.depth[u] = level + 1;
+        verts += 1;
+        edges += a.off[u + 1] - a.off[u];
+      }
+      if (lane == 0) next[w] = seen | fresh;
+    }
+  } else {
+    const uint64_t  count = min(l.entries, (unsigned long long)a.qcap);
+    const uint64_t* qi    = a.q[q];
+    uint64_t* const qo    = a.q[q ^ 1];
+    for (uint64_t i0 = warp * 4; i0 < count; i0 += nwarp * 4) {  // four entries per warp, eight lanes each
+      const uint64_t i = i0 + (lane >> 3);
+      uint64_t       e = 0, end = 0;
+      if (i < count) {
+        const uint64_t ent = qi[i];
+        const uint64_t ob  = a.off[ent >> 32];
+        const uint64_t at  = ob + (uint64_t)(uint32_t)ent * kVPiece;
+        e                  = at + (lane & 7);
+        end                = min(a.off[(ent >> 32) + 1], at + kVPiece);
+      }
+      while (__any_sync(kFullMask, e < end)) {
+        uint32_t x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = e + 8 * k < end ? __ldg(a.col + e + 8 * k) : kUnset;
+        bool won[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t bit = 1u << (x[k] & 31);
+          // a stale word only costs an atomic: bits go from 0 to 1
+          won[k] = x[k] != kUnset && !(cur[x[k] >> 5] & bit) && !(atomicOr(cur + (x[k] >> 5), bit) & bit);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (!__any_sync(kFullMask, won[k])) continue;
+          uint64_t deg = 0;
+          if (won[k]) {
+            a.depth[x[k]] = level + 1;
+            deg           = a.off[x[k] + 1] - a.off[x[k]];
+            verts += 1;
+            edges += deg;
+          }
+          v_append(a, qo, &nl.entries, won[k], x[k], deg);
+        }
+        e += 32;
       }
     }
   }
+  const unsigned long long vs = v_block_sum(verts), es = v_block_sum(edges);
+  if (threadIdx.x == 0 && vs) {
+    atomicAdd(&nl.verts, vs);
+    atomicAdd(&nl.edges, es);
+  }
 }
 
-// The per-vertex checks.  Lanes take consecutive vertices and scan up to 32
-// in-neighbours alone; longer in-lists are scanned by the whole warp.
-__global__ void __launch_bounds__(kVThreads) k_v_check(const uint64_t* __restrict__ in_off,
-                                                       const uint32_t* __restrict__ in_col,
-                                                       const uint32_t* __restrict__ depth,
-                                                       const uint32_t* __restrict__ parent, uint64_t n,
-                                                       uint32_t source, VerifyCounters* cnt) {
-  const unsigned     lane   = threadIdx.x & 31;
-  const uint64_t     stride = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t     n_up   = (n + 31) & ~31ull;
+// The next batch of levels starts from the last one's result.
+__global__ void k_v_carry(VerifyCounters* cnt) {
+  const VerifyLevel last = cnt->lv[kVBatch];
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i <= kVBatch; i += blockDim.x) cnt->lv[i] = i ? VerifyLevel{} : last;
+}
+
+__device__ __forceinline__ void v_fail(VerifyCounters* cnt, uint64_t u, uint32_t reason) {
+  atomicMin(&cnt->first, ((unsigned long long)u << 3) | reason);
+}
+
+// The per-vertex checks (reasons: 1 source wrong, 2 wrong depths, 3 no edge
+// from the parent, 4 reachability).  Lanes take consecutive vertices and scan
+// up to kVLane in-neighbours alone, kVProbe per round; the warp scans up to
+// kVHub more of a longer list; what is left is put down in pieces for
+// k_v_pieces.  piece: room for m / kVHub + the number of such lists.
+__global__ void __launch_bounds__(kVThreads) k_v_check(VerifyArgs a, const uint32_t* __restrict__ parent,
+                                                       uint32_t source, uint64_t* piece) {
+  const unsigned     lane    = threadIdx.x & 31;
+  const uint64_t     stride  = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t     n_up    = (a.n + 31) & ~31ull;
   unsigned long long reached = 0;
   for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n_up; u += stride) {
-    const bool     valid = u < n;
-    const uint32_t du    = valid ? depth[u] : kUnset;
+    const bool     valid = u < a.n;
+    const uint32_t du    = valid ? a.depth[u] : kUnset;
     const uint32_t pu    = valid ? parent[u] : kUnset;
-    uint32_t       fail  = 0;  // reason: 1 source wrong, 2 wrong depths, 3 no edge from the parent, 4 reachability
+    uint32_t       fail  = 0;
     bool           need  = false;  // parent search still open
     uint64_t       e = 0, end = 0;
     if (valid) {
@@ -104,49 +321,102 @@ __global__ void __launch_bounds__(kVThreads) k_v_check(const uint64_t* __restric
         if (u == source) {
           if (!(pu == u && du == 0)) fail = 1;
         } else {
-          e    = in_off[u];
-          end  = in_off[u + 1];
+          e    = a.in_off[u];
+          end  = a.in_off[u + 1];
           need = true;
         }
       } else if (du != pu) {
         fail = 4;
       }
     }
-    // lane scan of the first 32 in-neighbours
-    bool found = false;
-    if (need) {
-      const uint64_t lim = min(end, e + 32);
-      for (; e < lim; ++e)
-        if (in_col[e] == pu) {
-          found = true;
-          break;
-        }
-      if (found) need = false;
+    const bool search = need;
+    bool       found  = false;
+    {
+      const uint64_t lim = min(end, e + kVLane);
+      while (need && e < lim) {
+#pragma unroll
+        for (uint32_t k = 0; k < kVProbe; ++k)
+          if (e + k < lim && __ldg(a.in_col + e + k) == pu) found = true;
+        e = min(lim, e + kVProbe);
+        if (found) need = false;
+      }
     }
-    // the rest of long in-lists: the warp scans them together
     unsigned pend = __ballot_sync(kFullMask, need && e < end);
+    bool     open = false;  // the grid scans the rest
     while (pend) {
-      const int      ld = __ffs(pend) - 1;
+      const int ld = __ffs(pend) - 1;
       pend &= pend - 1;
-      const uint64_t b  = __shfl_sync(kFullMask, e, ld);
-      const uint64_t en = __shfl_sync(kFullMask, end, ld);
-      const uint32_t pp = __shfl_sync(kFullMask, pu, ld);
+      const uint64_t b   = __shfl_sync(kFullMask, e, ld);
+      const uint64_t en  = __shfl_sync(kFullMask, end, ld);
+      const uint32_t pp  = __shfl_sync(kFullMask, pu, ld);
+      const uint64_t lim = min(en, b + kVHub);
       bool           hit = false;
-      for (uint64_t base = b; base < en && !hit; base += 32) {
-        const uint64_t i = base + lane;
-        hit              = __any_sync(kFullMask, i < en && in_col[i] == pp);
+      for (uint64_t base = b; base < lim && !hit; base += 32 * kVProbe) {
+#pragma unroll
+        for (uint32_t k = 0; k < kVProbe; ++k) {
+          const uint64_t i = base + k * 32 + lane;
+          if (i < lim && __ldg(a.in_col + i) == pp) hit = true;
+        }
+        hit = __any_sync(kFullMask, hit);
+      }
+      if (!hit && lim < en) {
+        const uint64_t     np = (en - lim + kVHub - 1) / kVHub;
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(&a.cnt->pieces, (unsigned long long)np);
+        at                = __shfl_sync(kFullMask, at, 0);
+        const uint64_t us = __shfl_sync(kFullMask, u, ld);
+        for (uint64_t j = lane; j < np; j += 32) piece[at + j] = (us << 32) | j;
+        if ((int)lane == ld) open = true;
       }
       if ((int)lane == ld) found = hit;
     }
-    if (valid && du != kUnset && pu != kUnset && u != source) {
+    if (search && !open) {
       if (!found) fail = 3;
-      else if (du == 0 || depth[pu] != du - 1) fail = 2;  // the parent's depth (bfs.hpp:79)
+      else if (du == 0 || a.depth[pu] != du - 1) fail = 2;  // the parent's depth (bfs.hpp:79)
     }
-    if (fail) atomicMin(&cnt->first, ((unsigned long long)u << 3) | fail);
+    if (fail) v_fail(a.cnt, u, fail);
   }
+  const unsigned long long r = v_block_sum(reached);
+  if (threadIdx.x == 0 && r) atomicAdd(&a.cnt->reached, r);
+}
+
+// A warp per piece of a long in-list: a hit sets the vertex's bit in
+// `found` (all zero before).
+__global__ void __launch_bounds__(kVThreads) k_v_pieces(VerifyArgs a, const uint32_t* __restrict__ parent,
+                                                        const uint64_t* __restrict__ piece, uint32_t* found) {
+  const unsigned lane   = threadIdx.x & 31;
+  const uint64_t count  = a.cnt->pieces;
+  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += nwarps) {
+    const uint64_t u   = piece[i] >> 32;
+    const uint64_t en  = a.in_off[u + 1];
+    const uint64_t b   = a.in_off[u] + kVLane + kVHub + (piece[i] & 0xFFFFFFFFull) * kVHub;
+    const uint64_t lim = min(en, b + kVHub);
+    const uint32_t pp  = parent[u];
+    bool           hit = false;
+    for (uint64_t base = b; base < lim && !hit; base += 32 * kVProbe) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) reached += __shfl_xor_sync(kFullMask, reached, o);
-  if (lane == 0 && reached) atomicAdd(&cnt->reached, reached);
+      for (uint32_t k = 0; k < kVProbe; ++k) {
+        const uint64_t j = base + k * 32 + lane;
+        if (j < lim && __ldg(a.in_col + j) == pp) hit = true;
+      }
+      hit = __any_sync(kFullMask, hit);
+    }
+    if (hit && lane == 0) atomicOr(found + (u >> 5), 1u << (u & 31));
+  }
+}
+
+// The verdict of every vertex that was put down in pieces.
+__global__ void k_v_verdicts(VerifyArgs a, const uint32_t* __restrict__ parent, const uint64_t* __restrict__ piece,
+                             const uint32_t* __restrict__ found) {
+  const uint64_t count = a.cnt->pieces;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
+    if (piece[i] & 0xFFFFFFFFull) continue;
+    const uint64_t u  = piece[i] >> 32;
+    const uint32_t du = a.depth[u];
+    if (!((found[u >> 5] >> (u & 31)) & 1u)) v_fail(a.cnt, u, 3);
+    else if (du == 0 || a.depth[parent[u]] != du - 1) v_fail(a.cnt, u, 2);
+  }
 }
 
 int grid_v(const GraphDev* g, uint64_t items, uint64_t per_block) {
@@ -154,77 +424,156 @@ int grid_v(const GraphDev* g, uint64_t items, uint64_t per_block) {
   return (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)g->sm_count * 8, want));
 }
 
-struct VerifyBuffers {
-  uint32_t*       depth = nullptr;
-  uint32_t*       q[2]  = {nullptr, nullptr};
-  uint32_t*       par   = nullptr;  // device copy of host parents
-  VerifyCounters* cnt   = nullptr;
-  cudaStream_t    s     = nullptr;
+}  // namespace
+
+namespace nwg {
+
+// The check's state, made on a graph's first verification and kept with it
+// (making and freeing it took 2 ms of a call); calls on one graph take turns.
+struct VerifyWs {
+  std::mutex      mu;
+  bool            ready   = false;
+  uint32_t*       depth   = nullptr;
+  uint32_t*       vis     = nullptr;  // both copies
+  uint64_t*       q       = nullptr;  // both queues; the pieces of long in-lists after the traversal
+  uint32_t*       par     = nullptr;  // device copy of host parents, made when first needed
+  VerifyCounters* cnt     = nullptr;
+  VerifyCounters* cnt_host = nullptr;  // pinned
+  cudaStream_t    s       = nullptr;
   cudaEvent_t     ev0 = nullptr, ev1 = nullptr;
-  ~VerifyBuffers() {
-    if (s) cudaStreamSynchronize(s);
-    cudaFree(depth);
-    cudaFree(q[0]);
-    cudaFree(q[1]);
-    cudaFree(par);
-    cudaFree(cnt);
-    if (ev0) cudaEventDestroy(ev0);
-    if (ev1) cudaEventDestroy(ev1);
-    if (s) cudaStreamDestroy(s);
-  }
 };
 
-int verify(GraphDev* g, uint32_t source, const uint32_t* parents_host, const uint32_t* parents_dev,
-           nwg_verify_result* out) {
-  const uint64_t n = g->n;
-  VerifyBuffers  b;
-  if (cudaMalloc(&b.depth, std::max<uint64_t>(n, 1) * 4) != cudaSuccess ||
-      cudaMalloc(&b.q[0], std::max<uint64_t>(n, 1) * 4) != cudaSuccess ||
-      cudaMalloc(&b.q[1], std::max<uint64_t>(n, 1) * 4) != cudaSuccess ||
-      cudaMalloc(&b.cnt, sizeof(VerifyCounters)) != cudaSuccess ||
-      (parents_host && cudaMalloc(&b.par, std::max<uint64_t>(n, 1) * 4) != cudaSuccess)) {
+void verify_ws_free(VerifyWs* b) {
+  if (!b) return;
+  if (b->s) cudaStreamSynchronize(b->s);
+  cudaFree(b->depth);
+  cudaFree(b->vis);
+  cudaFree(b->q);
+  cudaFree(b->par);
+  cudaFree(b->cnt);
+  if (b->cnt_host) cudaFreeHost(b->cnt_host);
+  if (b->ev0) cudaEventDestroy(b->ev0);
+  if (b->ev1) cudaEventDestroy(b->ev1);
+  if (b->s) cudaStreamDestroy(b->s);
+  delete b;
+}
+
+}  // namespace nwg
+
+namespace {
+
+uint64_t queue_cap(const GraphDev* g) { return g->n + g->m / 512 + 1; }
+
+int verify_ws_make(const GraphDev* g, VerifyWs& b) {
+  const uint64_t n = std::max<uint64_t>(g->n, 1);
+  // the pieces need m / kVHub entries plus one per list of over kVHub: at most twice that
+  const uint64_t q = std::max<uint64_t>(2 * queue_cap(g), 2 * (g->in_m / kVHub) + 2);
+  if ((!b.depth && cudaMalloc(&b.depth, n * 4) != cudaSuccess) ||
+      (!b.vis && cudaMalloc(&b.vis, 2 * ((n + 31) / 32) * 4) != cudaSuccess) ||
+      (!b.q && cudaMalloc(&b.q, q * 8) != cudaSuccess) ||
+      (!b.cnt && cudaMalloc(&b.cnt, sizeof(VerifyCounters)) != cudaSuccess) ||
+      (!b.cnt_host && cudaMallocHost(&b.cnt_host, sizeof(VerifyCounters)) != cudaSuccess)) {
     cudaGetLastError();
+    return set_error(NWG_ENOMEM, "verifier allocation failed (n=" + std::to_string(g->n) + ")");
+  }
+  if (!b.s) NWG_CUDA_TRY(cudaStreamCreateWithFlags(&b.s, cudaStreamNonBlocking));
+  if (!b.ev0) NWG_CUDA_TRY(cudaEventCreate(&b.ev0));
+  if (!b.ev1) NWG_CUDA_TRY(cudaEventCreate(&b.ev1));
+  b.ready = true;
+  return NWG_OK;
+}
+
+int verify_on(GraphDev* g, VerifyWs& b, uint32_t source, const uint32_t* parents_host, const uint32_t* parents_dev,
+              nwg_verify_result* out) {
+  const uint64_t n = g->n;
+  if (!b.ready) {
+    const int rc = verify_ws_make(g, b);
+    if (rc) return rc;
+  }
+  if (parents_host && !b.par && cudaMalloc(&b.par, std::max<uint64_t>(n, 1) * 4) != cudaSuccess) {
+    cudaGetLastError();
+    b.par = nullptr;
     return set_error(NWG_ENOMEM, "verifier allocation failed (n=" + std::to_string(n) + ")");
   }
-  NWG_CUDA_TRY(cudaStreamCreateWithFlags(&b.s, cudaStreamNonBlocking));
-  NWG_CUDA_TRY(cudaEventCreate(&b.ev0));
-  NWG_CUDA_TRY(cudaEventCreate(&b.ev1));
+  VerifyArgs a;
+  a.off    = g->off;
+  a.col    = g->col;
+  a.in_off = g->in_off;
+  a.in_col = g->in_col;
+  a.n      = n;
+  a.m      = g->m;
+  a.depth  = b.depth;
+  a.vis[0] = b.vis;
+  a.vis[1] = b.vis + (n + 31) / 32;
+  a.q[0]   = b.q;
+  a.q[1]   = b.q + queue_cap(g);
+  a.qcap   = queue_cap(g);
+  a.cnt    = b.cnt;
   NWG_CUDA_TRY(cudaEventRecord(b.ev0, b.s));
   const uint32_t* par = parents_dev;
   if (parents_host) {
     NWG_CUDA_TRY(cudaMemcpyAsync(b.par, parents_host, n * 4, cudaMemcpyHostToDevice, b.s));
     par = b.par;
   }
-  k_v_init<<<grid_v(g, n, kVThreads), kVThreads, 0, b.s>>>(b.depth, n, source, b.q[0], b.cnt);
-  NWG_CUDA_TRY(cudaGetLastError());
-  uint64_t qsize = 1;
-  uint32_t level = 0;
-  unsigned long long next = 0;
-  while (qsize) {
-    NWG_CUDA_TRY(cudaMemsetAsync(&b.cnt->next, 0, sizeof(unsigned long long), b.s));
-    k_v_level<<<grid_v(g, qsize, kVThreads / 32), kVThreads, 0, b.s>>>(g->off, g->col, b.depth, b.q[level & 1],
-                                                                        qsize, b.q[(level + 1) & 1], n, level, b.cnt);
+  NWG_CUDA_TRY(cudaMemsetAsync(b.cnt, 0, sizeof(VerifyCounters), b.s));
+  k_v_init<<<grid_v(g, n, kVThreads), kVThreads, 0, b.s>>>(a, source);
+  const int gw = grid_v(g, std::max(n, g->m / kVPiece), kVThreads);  // a step's grid: levels of any size
+  uint32_t  base = 0;  // depth of the batch's first level, lv[0]
+  uint32_t  levels = 0;
+  // the first read-back after eight levels (hub graphs have 5-9), then every kVBatch
+  for (uint32_t done = 0, until = 8;;) {
+    for (; done < until; ++done) {
+      const uint32_t level = base + done;
+      k_v_queue<<<gw, kVThreads, 0, b.s>>>(a, done, level & 1);
+      k_v_step<<<gw, kVThreads, 0, b.s>>>(a, done, level & 1, level);
+    }
     NWG_CUDA_TRY(cudaGetLastError());
-    NWG_CUDA_TRY(cudaMemcpyAsync(&next, &b.cnt->next, sizeof next, cudaMemcpyDeviceToHost, b.s));
+    NWG_CUDA_TRY(cudaMemcpyAsync(b.cnt_host, b.cnt, sizeof(VerifyCounters), cudaMemcpyDeviceToHost, b.s));
     NWG_CUDA_TRY(cudaStreamSynchronize(b.s));
-    qsize = std::min<uint64_t>(next, n);
-    ++level;
+    if (b.cnt_host->lv[done].verts == 0) {
+      while (b.cnt_host->lv[done].verts == 0) --done;  // lv[0] holds a vertex
+      levels = base + done + 1;
+      break;
+    }
+    if (done == kVBatch) {
+      k_v_carry<<<1, 64, 0, b.s>>>(b.cnt);
+      base += kVBatch;
+      done = 0;
+    }
+    until = kVBatch;
   }
-  k_v_check<<<grid_v(g, n, kVThreads), kVThreads, 0, b.s>>>(g->in_off, g->in_col, b.depth, par, n, source, b.cnt);
+  // found bits of the long lists: the first bitmap copy, free now
+  const uint64_t words = (n + 31) / 32;
+  NWG_CUDA_TRY(cudaMemsetAsync(b.vis, 0, words * 4, b.s));
+  k_v_check<<<grid_v(g, n, kVThreads), kVThreads, 0, b.s>>>(a, par, source, b.q);
+  k_v_pieces<<<grid_v(g, g->in_m / kVHub, kVThreads / 32), kVThreads, 0, b.s>>>(a, par, b.q, b.vis);
+  k_v_verdicts<<<grid_v(g, g->in_m / kVHub, kVThreads), kVThreads, 0, b.s>>>(a, par, b.q, b.vis);
   NWG_CUDA_TRY(cudaGetLastError());
   NWG_CUDA_TRY(cudaEventRecord(b.ev1, b.s));
-  VerifyCounters hc;
-  NWG_CUDA_TRY(cudaMemcpyAsync(&hc, b.cnt, sizeof hc, cudaMemcpyDeviceToHost, b.s));
+  NWG_CUDA_TRY(cudaMemcpyAsync(b.cnt_host, b.cnt, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, b.s));
   NWG_CUDA_TRY(cudaStreamSynchronize(b.s));
-  nwg_verify_result r = {};
-  r.valid             = hc.first == ~0ull ? 1 : 0;
-  r.reason            = r.valid ? 0u : (uint32_t)(hc.first & 7u);
-  r.first_bad         = r.valid ? ~0ull : (hc.first >> 3);
-  r.reached           = hc.reached;
-  r.levels            = level;
+  const VerifyCounters& hc = *b.cnt_host;
+  nwg_verify_result     r  = {};
+  r.valid                  = hc.first == ~0ull ? 1 : 0;
+  r.reason                 = r.valid ? 0u : (uint32_t)(hc.first & 7u);
+  r.first_bad              = r.valid ? ~0ull : (hc.first >> 3);
+  r.reached                = hc.reached;
+  r.levels                 = levels;
   cudaEventElapsedTime(&r.device_ms, b.ev0, b.ev1);
   *out = r;
   return NWG_OK;
+}
+
+int verify(GraphDev* g, uint32_t source, const uint32_t* parents_host, const uint32_t* parents_dev,
+           nwg_verify_result* out) {
+  VerifyWs* b = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g->mu);
+    if (!g->verify_ws) g->verify_ws = new VerifyWs();
+    b = g->verify_ws;
+  }
+  std::lock_guard<std::mutex> lk(b->mu);
+  return verify_on(g, *b, source, parents_host, parents_dev, out);
 }
 
 }  // namespace
