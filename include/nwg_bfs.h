@@ -356,7 +356,9 @@ int nwg_bfs_noalloc(const uint64_t* out_off, const uint32_t* out_col, const uint
  * with double path counts, then float dependencies accumulated deepest
  * level first, every reached vertex (the source included) adding its own;
  * scores divided by the largest when normalize != 0.  `lanes` sources run
- * at once (0 = 4, at most 16), one stream each.  Scores (n floats) go to
+ * at once (0 = 4, at most 16), one stream each; their state (28 n bytes a
+ * lane, when that is at most 1 GB in all) is kept with the graph, and calls on
+ * one graph take turns.  Scores (n floats) go to
  * scores_host and/or scores_dev; float sums across sources, as in the
  * reference, so results agree with it within the reference verifier's
  * tolerance (1e-6 on normalized scores), not bit for bit. */

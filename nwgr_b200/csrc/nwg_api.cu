@@ -109,6 +109,8 @@ void graph_free(GraphDev* g) {
   g->roots_pool = nullptr;
   verify_ws_free(g->verify_ws);
   g->verify_ws = nullptr;
+  bc_ws_free(g->bc_ws);
+  g->bc_ws = nullptr;
   if (g->owns_out) {
     cudaFree(g->off);
     cudaFree(g->col);

@@ -295,6 +295,7 @@ struct GraphDev {
   Workspace*                default_ws = nullptr;
   Workspace*                pipe_ws    = nullptr;  // second lane of nwg_bfs_roots
   struct VerifyWs*          verify_ws  = nullptr;  // state of nwg_verify
+  struct BcWs*              bc_ws      = nullptr;  // state of nwg_bc
   struct RootsPool*         roots_pool = nullptr;  // its rows and queues where blocks take the roots
   std::vector<Workspace*>   workspaces;
   std::vector<MsWorkspace*> ms_workspaces;
@@ -340,8 +341,9 @@ int  run_traversal(const DobfsParams& params, int sm_count, uint32_t root, int a
                    void* q, cudaStream_t stream);
 int  zero_indegree_packed(RaggedDev* r);
 
-// nwg_verify.cu
+// nwg_verify.cu, nwg_bc.cu
 void verify_ws_free(struct VerifyWs* b);
+void bc_ws_free(struct BcWs* w);
 
 // nwg_msbfs.cu
 int      ms_ws_init(GraphDev* g, MsWorkspace* ws);
