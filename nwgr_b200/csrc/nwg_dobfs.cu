@@ -136,9 +136,7 @@ struct StepView {
   uint32_t*           qbig;     // chunked vertices appended
   uint32_t*           nhub;     // deferred hub records appended
   unsigned long long* scout;    // out-degree sum of the vertices a top-down step discovers
-  unsigned long long* awake;    // vertices a pull discovers
-  uint32_t*           mark;     // top-down step: NULL = queue the discoveries, else set their bits here
-  uint32_t            mark_deg; // marking step: also sum the discoveries' out-degrees into scout
+  unsigned long long* awake;    // vertices a pull or a marking step discovers
 };
 
 // ---------------------------------------------------------------------------
@@ -417,6 +415,50 @@ __device__ __forceinline__ void flush_winners(const DobfsParams& p, const StepVi
   __syncwarp();
 }
 
+// End of a step in which the block has at most kLight buffered winners and
+// nothing was flushed before: a thread per winner, appended by warp.  One
+// barrier instead of a dozen, and one vertex per thread instead of one per
+// warp's buffer: a block of a small frontier spent 4-5 of a step's 14 us in
+// the general flush.  Block-uniform; returns false (and has done nothing)
+// where the general flush is needed.
+constexpr uint32_t kLight = 64;
+template <bool kDefer>
+__device__ __forceinline__ bool flush_light(const DobfsParams& p, const StepView& sv, const TdWarp* tws, uint32_t wcnt,
+                                            bool pending) {
+  __shared__ uint32_t s_cnt[kWarps];
+  const bool          any = __any_sync(kFullMask, pending);
+  if ((threadIdx.x & 31) == 0) s_cnt[threadIdx.x >> 5] = any ? kLight + 1 : wcnt;
+  __syncthreads();
+  uint32_t total = 0, src = 0, at = threadIdx.x;  // this thread's winner: entry `at` of warp src's buffer
+#pragma unroll
+  for (uint32_t w = 0; w < kWarps; ++w) {
+    const uint32_t c = s_cnt[w];
+    total += c;
+    if (src == w && at >= c) {
+      at -= c;
+      ++src;
+    }
+  }
+  if (total > kLight) return false;
+  if ((threadIdx.x & ~31u) < total) {  // whole warps
+    const bool     mine = threadIdx.x < total;
+    const uint32_t v[1] = {mine ? tws[src].win[at] : 0u};
+    uint64_t       d[1] = {0};
+    uint32_t       nbig = 0;
+    out_degrees<1>(p, v, mine ? 1u : 0u, d);
+    append_warp<1, kDefer>(p, sv, v, d, mine ? 1u : 0u, nbig);
+    unsigned long long scout = d[0];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) scout += __shfl_xor_sync(kFullMask, scout, o);
+    nbig = __reduce_add_sync(kFullMask, nbig);
+    if ((threadIdx.x & 31) == 0) {
+      if (scout) atomicAdd(sv.scout, scout);
+      if (nbig) atomicAdd(sv.qbig, nbig);
+    }
+  }
+  return true;
+}
+
 // End of a step: every warp's remaining buffered winners are appended with
 // one reservation for the whole block.  All threads of the block call.
 template <bool kDefer>
@@ -478,25 +520,13 @@ __device__ __forceinline__ void visit_batch(const DobfsParams& p, const StepView
 #pragma unroll
   for (int k = 0; k < kVisit; ++k)
     if ((try_mask & (1u << k)) && !(old[k] & (1u << (v[k] & 31)))) win |= 1u << k;
-  const uint32_t cnt = __popc(win);
-  if (kMark) {  // marking step: the bit is the discovery record; no queue entry
+  if (kMark) {
 #pragma unroll
-    for (int k = 0; k < kVisit; ++k) {
-      if (win & (1u << k)) {
-        parents[v[k]] = u[k];
-        atomicOr(sv.mark + (v[k] >> 5), 1u << (v[k] & 31));
-      }
-    }
-    nbig += cnt;  // discoveries
-    if (sv.mark_deg) {  // a marking top-down step also sums their out-degrees (bfs.hpp:286)
-      uint64_t d[kVisit];
-      out_degrees<kVisit>(p, v, win, d);
-#pragma unroll
-      for (int k = 0; k < kVisit; ++k)
-        if (win & (1u << k)) scout += d[k];
-    }
+    for (int k = 0; k < kVisit; ++k)
+      if (win & (1u << k)) parents[v[k]] = u[k];
     return;
   }
+  const uint32_t cnt = __popc(win);
   const uint32_t inc = warp_incl_scan(cnt);
   const uint32_t tot = __shfl_sync(kFullMask, inc, 31);
   if (tot == 0) return;
@@ -746,11 +776,13 @@ __device__ __forceinline__ uint32_t td_kernel_setup(CtrlHdr& c) {
 // Discoveries are estimated as the front's out-edges times the unvisited
 // share, at most the candidates, and, on graphs of average degree <= 8
 // (meshes and roads, whose fronts are bands), at most twice the front.
-__device__ __forceinline__ uint64_t active_vertices(const DobfsParams& p) {
-  return p.n > p.nzero ? p.n - p.nzero : 1;  // vertices with edges
+__host__ __device__ __forceinline__ void set_density(DobfsParams& p) {
+  p.active  = p.n > p.nzero ? p.n - p.nzero : 1;  // vertices with edges
+  p.avg_deg = p.m / p.active > 1 ? p.m / p.active : 1;
 }
-__device__ __forceinline__ uint64_t avg_degree(const DobfsParams& p) {
-  return max((uint64_t)1, p.m / active_vertices(p));
+// a > b / c for integers (c > 0) without the division: exactly a * c > b.
+__device__ __forceinline__ bool over_quotient(uint64_t a, uint64_t b, uint64_t c) {
+  return __umul64hi(a, c) != 0 || a * c > b;
 }
 __device__ __forceinline__ uint64_t pull_candidates(const DobfsParams& p, uint64_t reached) {
   const uint64_t excl = p.nzero + reached;
@@ -761,8 +793,8 @@ __device__ __forceinline__ uint64_t pull_candidates(const DobfsParams& p, uint64
 __device__ __forceinline__ uint64_t est_wins(const DobfsParams& p, uint64_t reached, uint64_t front,
                                              uint64_t front_edges) {
   const uint64_t cand = pull_candidates(p, reached);
-  uint64_t wins = min(cand, (uint64_t)((double)front_edges * (double)cand / (double)active_vertices(p)));
-  if (avg_degree(p) <= 8) wins = min(wins, 2 * front);
+  uint64_t wins = min(cand, (uint64_t)((double)front_edges * (double)cand / (double)p.active));
+  if (p.avg_deg <= 8) wins = min(wins, 2 * front);
   return wins;
 }
 __device__ __forceinline__ bool push_cheaper(const DobfsParams& p, uint64_t reached, uint64_t front,
@@ -770,7 +802,7 @@ __device__ __forceinline__ bool push_cheaper(const DobfsParams& p, uint64_t reac
   if (!p.symmetric || front_edges == 0) return false;
   const uint64_t cand   = pull_candidates(p, reached);
   const uint64_t wins   = est_wins(p, reached, front, front_edges);
-  const uint64_t t      = max((uint64_t)1, min(avg_degree(p), p.m / front_edges));
+  const uint64_t t      = max((uint64_t)1, min(p.avg_deg, p.m / front_edges));
   const uint64_t push   = 300 * front + 50 * front_edges + 500 * wins;
   const uint64_t pull   = 26 * p.n + cand * (30 * t + 30 * t * t / 16);
   return push < pull;
@@ -793,11 +825,11 @@ __device__ __forceinline__ bool pull_as_push(const DobfsParams& p, const CtrlHdr
 // bitmap, as after any pull (bfs.hpp:235-239).
 __device__ __forceinline__ bool mark_push(const DobfsParams& p, const CtrlHdr& c, uint64_t front,
                                           uint64_t front_edges) {
-  if (!c.mark_ok) return false;
-  const uint64_t wins = est_wins(p, c.reached, front, front_edges);
+  if (!c.mark_ok || front_edges < p.n / 32) return false;
+  const uint64_t wins = est_wins(p, c.reached, front, front_edges);  // at most front_edges
   if (wins < p.n / 32) return false;
   if (!(wins >= front || wins > p.n / c.beta)) return false;
-  return !push_cheaper(p, c.reached + wins, wins, wins * avg_degree(p));
+  return !push_cheaper(p, c.reached + wins, wins, wins * p.avg_deg);
 }
 
 // A top-down step after which the reference's rule will very likely switch
@@ -810,10 +842,10 @@ __device__ __forceinline__ bool mark_push(const DobfsParams& p, const CtrlHdr& c
 // traversal top-down, bitmap -> queue rebuilds the queue from C0 first.
 __device__ __forceinline__ bool mark_td(const DobfsParams& p, const CtrlHdr& c, uint64_t front,
                                         uint64_t front_edges) {
-  if (!c.mark_ok || c.topdown_only) return false;
+  if (!c.mark_ok || c.topdown_only || front_edges < p.n / 32) return false;
   const uint64_t wins = est_wins(p, c.reached, front, front_edges);
   if (wins < p.n / 32) return false;
-  const uint64_t scout = wins * avg_degree(p);
+  const uint64_t scout = wins * p.avg_deg;
   if (scout / 2 <= c.edges_to_check / c.alpha) return false;
   return !push_cheaper(p, c.reached + wins, wins, scout);
 }
@@ -843,10 +875,10 @@ __device__ __forceinline__ uint32_t mark_td_setup(CtrlHdr& c) {
 // line it reproduces.  Returns the next action (kActNone when the traversal
 // is over).  It advances a copy `c` of the decision state; `writer` marks
 // the one caller that writes the trace.  It reads nothing else that changes
-// during a step except the sticky error word, so equal copies given equal
-// counters make equal decisions.
-__device__ uint32_t decide_on(const DobfsParams& p, CtrlHdr& c, bool writer, bool read_err = true) {
-  const unsigned long long now = globaltimer();
+// during a step, so equal copies given equal
+// counters make equal decisions.  err: the sticky error word.
+__device__ uint32_t decide_on(const DobfsParams& p, CtrlHdr& c, bool writer, int32_t err) {
+  const unsigned long long now = writer ? globaltimer() : 0ull;
   const uint64_t N    = p.n;
   uint32_t       next = kActNone;
   bool           done = false, queue_decision = false;
@@ -871,7 +903,7 @@ __device__ uint32_t decide_on(const DobfsParams& p, CtrlHdr& c, bool writer, boo
         c.reached += awake;
         c.cur = nxt;  // the discoveries, held as a queue, are the next front
         if (awake > 0) c.levels++;
-        if (awake >= c.old_awake || awake > N / c.beta) {  // bfs.hpp:229
+        if (awake >= c.old_awake || over_quotient(awake, N, c.beta)) {  // bfs.hpp:229
           c.old_awake   = awake;                           // bfs.hpp:206
           c.awake_count = awake;
           if (pull_as_push(p, c, awake, c.acc_scout)) {
@@ -922,7 +954,7 @@ __device__ uint32_t decide_on(const DobfsParams& p, CtrlHdr& c, bool writer, boo
         break;
       }
       c.levels++;
-      if (c.scout_count > c.edges_to_check / c.alpha) {  // bfs.hpp:186
+      if (over_quotient(c.scout_count, c.edges_to_check, c.alpha)) {  // bfs.hpp:186
         c.awake_count = nq;                                // bfs.hpp:199-202
         c.old_awake   = nq;
         // a pull over V (a push would need the queue; both discover the same set)
@@ -949,7 +981,7 @@ __device__ uint32_t decide_on(const DobfsParams& p, CtrlHdr& c, bool writer, boo
       c.reached += awake;
       c.bm ^= 1u;  // C[bm] now holds this pull's discoveries (the new "front")
       if (awake > 0) c.levels++;
-      if (awake >= c.old_awake || awake > N / c.beta) {  // bfs.hpp:229
+      if (awake >= c.old_awake || over_quotient(awake, N, c.beta)) {  // bfs.hpp:229
         c.old_awake   = awake;                           // bfs.hpp:206
         c.awake_count = awake;
         c.acc_awake   = 0;
@@ -983,7 +1015,7 @@ __device__ uint32_t decide_on(const DobfsParams& p, CtrlHdr& c, bool writer, boo
 
   if (queue_decision) {
     const uint64_t nq = frontier_size(c, c.cur);
-    if (!c.topdown_only && c.scout_count > c.edges_to_check / c.alpha) {  // bfs.hpp:186
+    if (!c.topdown_only && over_quotient(c.scout_count, c.edges_to_check, c.alpha)) {  // bfs.hpp:186
       c.awake_count = nq;                                                // bfs.hpp:199-202
       c.old_awake   = nq;
       if (pull_as_push(p, c, nq, c.scout_count)) {  // scout_count: the frontier's out-edges
@@ -1008,7 +1040,6 @@ __device__ uint32_t decide_on(const DobfsParams& p, CtrlHdr& c, bool writer, boo
   if (!done && ++c.steps > c.max_steps) {
     c.status = NWG_ETIMEDOUT;  // loop bound; a BFS needs at most ~2n actions
   }
-  const int32_t err = read_err ? *(volatile int32_t*)&p.ctrl->err : 0;
   if (c.status == 0 && err != 0) c.status = err;
   if (c.status != 0) done = true;
   c.action      = done ? kActNone : next;
@@ -1028,7 +1059,7 @@ __device__ uint32_t decide_core(const DobfsParams& p) {
 #pragma unroll
     for (int i = 0; i < kV; ++i) dst[i] = __ldcg(src + i);
   }
-  const uint32_t next = decide_on(p, c, true);
+  const uint32_t next = decide_on(p, c, true, *(volatile int32_t*)&p.ctrl->err);
   {
     const uint4* src = reinterpret_cast<const uint4*>(&c);
     uint4*       dst = reinterpret_cast<uint4*>(&p.ctrl->h);
@@ -1105,19 +1136,72 @@ __device__ __forceinline__ void td_step(const DobfsParams& p, const StepView& sv
     }
     gather_ranges<kDefer, kMark>(p, sv, u, lo, hi, tw, wcnt, scout, nbig);
   }
-  if (!kMark) flush_block<kDefer>(p, sv, tws, wcnt, scout, nbig, true);
+  if (kMark) return;
+  if (flush_light<kDefer>(p, sv, tws, wcnt, (scout | nbig) != 0)) return;
+  flush_block<kDefer>(p, sv, tws, wcnt, scout, nbig, true);
 
   const unsigned long long tot = block_sum(scout);
   __syncthreads();
-  const uint32_t nb = block_sum(nbig);  // a marking step: its discoveries
+  const uint32_t nb = block_sum(nbig);
   if (threadIdx.x == 0) {
     if (tot) atomicAdd(sv.scout, tot);
-    if (nb) {
-      if (kMark)
-        atomicAdd(sv.awake, (unsigned long long)nb);
-      else
-        atomicAdd(sv.qbig, nb);
+    if (nb) atomicAdd(sv.qbig, nb);
+  }
+}
+
+// The discoveries of a marking step: `mark` holds the visited bitmap as it
+// was before the step and gets the bits the step added; their count goes to
+// the awake count and, for a marking top-down step (deg), their out-degree
+// sum to scout (bfs.hpp:286).  The degrees are read in vertex order, 16 bytes
+// a lane (8 vertices, four lanes a word).  Setting a bit and looking a degree
+// up for each discovery as it is claimed costs two scattered L2 accesses
+// beside the claim and the parent: uniform 2^24's step of 13M discoveries
+// took 609 us that way, 458 us with this pass; RMAT-24's of 3M 168 and 152.
+// Steps without claims (each edge to an unvisited vertex stores its parent,
+// this pass reads the parents) took 440 and 196 us: not kept.
+// Not inlined: its registers would add to the step functions' spills.
+__device__ __noinline__ void mark_collect(const uint32_t* V, uint32_t* mark, uint64_t n, const uint16_t* deg16,
+                                          const uint64_t* off, bool deg, unsigned long long* awake_out,
+                                          unsigned long long* scout_out) {
+  const unsigned     lane   = threadIdx.x & 31;
+  const uint64_t     warp   = (uint64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
+  const uint64_t     nwarp  = (uint64_t)gridDim.x * kWarps;
+  const uint64_t     nwords = (n + 31) / 32;
+  unsigned long long found = 0, scout = 0;
+  for (uint64_t w0 = warp * 32; w0 < nwords; w0 += nwarp * 32) {  // 32 words: a lane each
+    const uint64_t w = w0 + lane;
+    uint32_t       x = 0;
+    if (w < nwords) {
+      x       = V[w] & ~mark[w];
+      mark[w] = x;
     }
+    found += __popc(x);
+    if (!deg) continue;
+#pragma unroll 4
+    for (uint32_t j = 0; j < 32; j += 8) {  // words j .. j + 7
+      const uint32_t y = __shfl_sync(kFullMask, x, j + (lane >> 2)) >> ((lane & 3) * 8) & 0xFFu;
+      if (!y) continue;
+      const uint64_t v0 = (w0 + j + (lane >> 2)) * 32 + (lane & 3) * 8;
+      if (deg16 && v0 + 8 <= n) {
+        const uint4    d  = __ldg(reinterpret_cast<const uint4*>(deg16 + v0));  // v0 is a multiple of 8
+        const uint32_t dd[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const uint32_t dk = (dd[k >> 1] >> (16 * (k & 1))) & 0xFFFFu;
+          if ((y >> k) & 1u) scout += dk != 0xFFFFu ? (uint64_t)dk : off[v0 + k + 1] - off[v0 + k];
+        }
+      } else {
+        for (int k = 0; k < 8; ++k)
+          if ((y >> k) & 1u) scout += off[v0 + k + 1] - off[v0 + k];
+      }
+    }
+  }
+  const unsigned long long nf = block_sum(found);
+  __syncthreads();
+  const unsigned long long ns = block_sum(scout);
+  if (threadIdx.x == 0) {
+    if (nf) atomicAdd(awake_out, nf);
+    if (ns) atomicAdd(scout_out, ns);
   }
 }
 
@@ -1139,8 +1223,6 @@ __device__ __forceinline__ StepView td_view(const DobfsParams& p) {
   sv.nhub          = &c->nhub[sv.out];
   sv.scout         = &c->acc_scout;
   sv.awake         = &c->acc_awake;
-  sv.mark          = nullptr;
-  sv.mark_deg      = 0;
   return sv;
 }
 
@@ -1158,8 +1240,6 @@ __device__ __forceinline__ StepView bu_view(const DobfsParams& p) {
   sv.nhub       = &c->nhub[sv.out];
   sv.scout      = &c->acc_scout;
   sv.awake      = &c->acc_awake;
-  sv.mark       = nullptr;
-  sv.mark_deg   = 0;
   return sv;
 }
 
@@ -1573,8 +1653,8 @@ __global__ void __launch_bounds__(kThreads) k_b2q(DobfsParams p) {
 // the decisions at the start of step - 1, which every block finished before
 // the barrier ending step - 1, and it is next written in step + 1, after the
 // barrier ending this step.  Deferred hub chunk entries are written by the
-// whole grid after the barrier and a second barrier orders them before the
-// next step reads the queue.  The steps are the level-loop kernels' own
+// whole grid after the next decision, if the step it chose expands them, and
+// a second barrier orders them before that step reads the queue.  The steps are the level-loop kernels' own
 // (td_step, bu_step, b2q_step); the barrier's arrival count is cleared by
 // the host before the launch.
 constexpr int kTravPerSm = 4;  // 64 registers: the top-down step does not spill
@@ -1582,38 +1662,40 @@ constexpr int kTravPerSm = 4;  // 64 registers: the top-down step does not spill
 // Grid barrier of k_trav: every block arrives (even after an error, so the
 // others are not left waiting); the wait is bounded like grid_barrier's.
 // The arrival count only grows during a launch (the host clears it before
-// each one): the block that makes the k-th arrival waits until the count
-// reaches the next multiple of nblocks.  Passing costs one atomic per block
-// and the polls; there is no reset or generation word to update, so the
-// last block to arrive releases the others with its own arrival.  The fence
-// before the arrival and the acquire loads of the count order every
-// block's writes before the barrier ahead of every read after it.
+// each one): barrier k is passed when the count reaches k * nblocks, which
+// each block keeps in `target` (shared, zero at the start, thread 0's).  So
+// an arrival needs no answer: it is one release reduction, and the block
+// polls at once; there is no reset or generation word, and the last block to
+// arrive releases the others with its own arrival.  The release orders the
+// block's writes (before the __syncthreads) ahead of the arrival, the acquire
+// loads of the count every read after it.  With a fence, an atomic that
+// returns the count and a fence after the wait a step's barrier took 1.9 us
+// beside the waiting, 0.8 us so.
 __device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long* a) {
   unsigned long long v;
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(a) : "memory");
   return v;
 }
 
-__device__ __forceinline__ bool trav_barrier(const DobfsParams& p, unsigned nblocks,
-                                             unsigned max_spins = kBarrierSpins, unsigned sleep_ns = 32) {
+__device__ __forceinline__ bool trav_barrier(const DobfsParams& p, unsigned nblocks, unsigned long long& target,
+                                             unsigned max_spins = kBarrierSpins) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned long long* cnt = &p.ctrl->bar.arrivals;
-    int                 ok  = 1;
-    __threadfence();
-    const unsigned long long k      = atomicAdd(cnt, 1ull);
-    const unsigned long long target = (k / nblocks + 1) * nblocks;
-    unsigned                 spins  = 0;
-    while (ld_acquire64(cnt) < target) {
+    unsigned long long* const cnt  = &p.ctrl->bar.arrivals;
+    const unsigned long long  want = target + nblocks;
+    target                         = want;
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(cnt), "l"(1ull) : "memory");
+    int      ok    = 1;
+    unsigned spins = 0;
+    while (ld_acquire64(cnt) < want) {
       if (++spins > max_spins) {
         atomicCAS(&p.ctrl->err, 0, NWG_ETIMEDOUT);
         ok = 0;
         break;
       }
-      __nanosleep(sleep_ns);
+      __nanosleep(32);
     }
-    __threadfence();
     s_ok = ok;
   }
   __syncthreads();
@@ -1860,7 +1942,7 @@ __device__ __forceinline__ void solo_run(const DobfsParams& p, CtrlHdr& c, SoloS
       c.qbig[nxt]        = 0;
       c.nhub[nxt]        = 0;
       c.acc_scout        = E;
-      const uint32_t next = decide_on(p, c, true, false);
+      const uint32_t next = decide_on(p, c, true, 0);
       *s_flag = (solo_ok(c, next) && lv + 1 < kSoloLevels) ? 1u : 0u;
     }
     __syncthreads();
@@ -1875,13 +1957,15 @@ __global__ void __launch_bounds__(kThreads, kTravPerSm)
   __shared__ StepShared sm;
   __shared__ CtrlHdr    s_c;  // this block's copy of the decision state
   __shared__ uint32_t   s_next;
+  __shared__ unsigned long long s_target;  // arrivals that pass the next barrier (thread 0's)
   constexpr int       kV = sizeof(CtrlHdr) / 16;
+  if (threadIdx.x == 0) s_target = 0;
   init_step(p, root, alpha, beta, parents, topdown_only, blockIdx.x, gridDim.x, false);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     for (int i = 0; i < 3; ++i) p.ctrl->acc[i] = StepAcc{};
     p.ctrl->kernels = 1;
   }
-  bool ok = trav_barrier(p, gridDim.x);
+  bool ok = trav_barrier(p, gridDim.x, s_target);
   if (ok && threadIdx.x == 0) {
     const uint4* src = reinterpret_cast<const uint4*>(&p.ctrl->h);
     uint4*       dst = reinterpret_cast<uint4*>(&s_c);
@@ -1902,25 +1986,29 @@ __global__ void __launch_bounds__(kThreads, kTravPerSm)
         }
         s_next = s_c.action;
       } else {
+        const int32_t err = __ldcg(&p.ctrl->err);  // loads beside the counters
         if (step > 0) {  // the previous step's counters, final after the barrier
-          const StepAcc* a = &p.ctrl->acc[(step - 1) % 3];
+          const StepAcc*           a  = &p.ctrl->acc[(step - 1) % 3];
+          const unsigned long long aq = __ldcg(&a->qpos), as = __ldcg(&a->scout), aa = __ldcg(&a->awake);
+          const uint32_t           ab = __ldcg(&a->qbig), ah = __ldcg(&a->nhub);
           if (last != kActBU && last != kActBUMark && last != kActTDMark) {
             const uint32_t ob = last == kActB2Q ? s_c.cur : (s_c.cur ^ 1u);  // the queue buffer it wrote
-            s_c.qpos[ob]      = __ldcg(&a->qpos);
-            s_c.qbig[ob]      = __ldcg(&a->qbig);
-            s_c.nhub[ob]      = __ldcg(&a->nhub);
+            s_c.qpos[ob]      = aq;
+            s_c.qbig[ob]      = ab;
+            s_c.nhub[ob]      = ah;
           }
-          s_c.acc_scout = __ldcg(&a->scout);
-          s_c.acc_awake = __ldcg(&a->awake);
+          s_c.acc_scout = as;
+          s_c.acc_awake = aa;
         }
-        s_next = decide_on(p, s_c, blockIdx.x == 0);
+        s_next = decide_on(p, s_c, blockIdx.x == 0, err);
       }
     }
     __syncthreads();
     const uint32_t next = s_next;
-    if (resume && next != kActNone && s_c.nhub[s_c.cur] != 0) {  // hub records of the solo frontier
+    if (next != kActNone && next != kActBU && next != kActB2Q && s_c.nhub[s_c.cur] != 0) {
+      // hub records of the frontier this step expands (nothing else reads the queue)
       expand_hubs(p, s_c.cur, s_c.nhub[s_c.cur], blockIdx.x, gridDim.x);
-      ok = trav_barrier(p, gridDim.x);
+      ok = trav_barrier(p, gridDim.x, s_target);
       if (!ok) break;
       if (threadIdx.x == 0) s_c.nhub[s_c.cur] = 0;
       __syncthreads();
@@ -1939,7 +2027,7 @@ __global__ void __launch_bounds__(kThreads, kTravPerSm)
           for (int i = 0; i < kV; ++i) dst[i] = src[i];
         }
       }
-      ok     = trav_barrier(p, gridDim.x);
+      ok     = trav_barrier(p, gridDim.x, s_target);
       resume = true;
       last   = kActNone;
       continue;
@@ -1953,16 +2041,14 @@ __global__ void __launch_bounds__(kThreads, kTravPerSm)
     sv.nhub    = &a->nhub;
     sv.scout   = &a->scout;
     sv.awake   = &a->awake;
-    sv.mark     = nullptr;
-    sv.mark_deg = next == kActTDMark ? 1u : 0u;
-    if (next == kActBUMark || next == kActTDMark) {
-      // the discovery bitmap is cleared by the whole grid before any claim
-      uint32_t* const cw = s_c.bm ? p.C0 : p.C1;
+    const bool      marking = next == kActBUMark || next == kActTDMark;
+    uint32_t* const mark    = s_c.bm ? p.C0 : p.C1;  // the discovery bitmap of a marking step
+    if (marking) {
+      // it takes the visited bitmap as it is before any claim
       for (uint64_t w = (uint64_t)blockIdx.x * kThreads + threadIdx.x; w < p.nwords; w += (uint64_t)gridDim.x * kThreads)
-        cw[w] = 0u;
-      ok = trav_barrier(p, gridDim.x);
+        mark[w] = p.V[w];
+      ok = trav_barrier(p, gridDim.x, s_target);
       if (!ok) break;
-      sv.mark = cw;
     }
     if (next == kActBU) {
       sv.in = sv.out = s_c.cur;
@@ -1978,20 +2064,18 @@ __global__ void __launch_bounds__(kThreads, kTravPerSm)
       const uint64_t q = s_c.qpos[s_c.cur];
       sv.nS          = min((uint64_t)(q & 0xFFFFFFFFull), p.qs_cap);
       sv.nC          = min((uint64_t)(q >> 32), p.qc_cap);
-      if (sv.mark)
+      if (marking) {
         td_step<true, true>(p, sv, sm.td.tw, blockIdx.x, gridDim.x);
-      else
+        ok = trav_barrier(p, gridDim.x, s_target);
+        if (!ok) break;
+        StepAcc* const acc = &p.ctrl->acc[step % 3];
+        mark_collect(p.V, s_c.bm ? p.C0 : p.C1, p.n, p.deg16, p.off, s_next == kActTDMark, &acc->awake, &acc->scout);
+      } else {
         td_step<true>(p, sv, sm.td.tw, blockIdx.x, gridDim.x);
-    }
-    ok = trav_barrier(p, gridDim.x);
-    if (ok && next != kActBU && next != kActB2Q && next != kActBUMark && next != kActTDMark) {
-      const uint32_t nh = __ldcg(&a->nhub);  // the same in every block after the barrier
-      if (nh) {
-        expand_hubs(p, sv.out, nh, blockIdx.x, gridDim.x);
-        ok = trav_barrier(p, gridDim.x);
       }
     }
-    last = next;
+    ok   = trav_barrier(p, gridDim.x, s_target);
+    last = s_next;  // from shared memory again: values kept across the step functions spill
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     const int32_t err = __ldcg(&p.ctrl->err);
@@ -2229,6 +2313,7 @@ __global__ void __launch_bounds__(kThreads) k_ragged(RaggedParams rp) {
     p.qc_cap               = L.qc_cap;
     p.th                   = Thresholds{item.warp_min, 256, 8};
     p.nzero                = 0;  // unknown here: the push-or-pull estimate then counts isolated vertices too
+    set_density(p);
     p.symmetric            = 1;  // packed graphs are symmetric
     p.ctrl                 = reinterpret_cast<Ctrl*>(slot + L.ctrl);
     init_step(p, item.root, (uint32_t)item.alpha, (uint32_t)item.beta, rp.parents + item.out_base, 0u, 0, 1);
@@ -2349,6 +2434,7 @@ int ws_init(GraphDev* g, Workspace* ws) {
   P.hub_cap      = hub_cap;
   P.th           = g->th;
   P.nzero        = g->nzero;
+  set_density(P);
   P.symmetric    = g->symmetric ? 1u : 0u;
   P.ctrl         = ws->ctrl;
   // every block of the persistent kernel must be resident (cooperative launch)
@@ -2496,6 +2582,7 @@ int run_traversal(const DobfsParams& params, int sm_count, uint32_t root, int al
     g.Z        = nullptr;  // not built
     return blk_one_launch(g, root, alpha, beta, parents, static_cast<BlkEnt*>(q), P.ctrl, false, stream);
   }
+  set_density(P);
   const int rc = zero_indegree_into(P.in_off, P.n, const_cast<uint32_t*>(P.Z), sm_count, stream);
   if (rc) return rc;
   uint32_t r = root, a = (uint32_t)alpha, b = (uint32_t)beta, td = 0u;
@@ -2883,7 +2970,9 @@ int ragged_launch(RaggedDev* r, uint32_t n_items, uint32_t n_big, uint32_t* pare
 // it.  Every block gives up after max_spins polls, records NWG_ETIMEDOUT and
 // returns -- the path a real barrier takes when a block never arrives.
 __global__ void k_wait_probe(DobfsParams p, unsigned max_spins) {
-  const bool ok = trav_barrier(p, gridDim.x + 1, max_spins);
+  __shared__ unsigned long long s_target;
+  if (threadIdx.x == 0) s_target = 0;
+  const bool ok = trav_barrier(p, gridDim.x + 1, s_target, max_spins);
   if (!ok && threadIdx.x == 0 && blockIdx.x == 0) p.ctrl->h.status = __ldcg(&p.ctrl->err);
 }
 

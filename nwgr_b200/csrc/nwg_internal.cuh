@@ -157,6 +157,7 @@ struct DobfsParams {
   uint64_t        hub_cap;
   Thresholds      th;
   uint64_t        nzero;      // vertices without in-edges (0 where unknown: only a cost estimate uses it)
+  uint64_t        active, avg_deg;  // vertices with edges, their average degree (at least 1): the estimate's
   uint32_t        symmetric;  // the in-CSR is the out-CSR (a pull may then run as a push)
   Ctrl*           ctrl;
 };
