@@ -277,15 +277,25 @@ int bfs_sync(GraphDev* g, uint32_t root, int alpha, int beta, uint32_t* parents_
   int                         rc = get_default_ws(g, &ws);
   if (rc) return rc;
   uint32_t* dst = parents_dev ? parents_dev : ws->parents;
-  NWG_CUDA_TRY(cudaEventRecord(ws->ev0, ws->stream));
-  rc = ws_launch(ws, root, alpha, beta, dst, ws->stream, topdown_only);
-  if (rc) return rc;
-  NWG_CUDA_TRY(cudaEventRecord(ws->ev1, ws->stream));
-  if (parents_host)
-    NWG_CUDA_TRY(cudaMemcpyAsync(parents_host, dst, g->n * sizeof(uint32_t), cudaMemcpyDeviceToHost, ws->stream));
-  const size_t ctrl_bytes = stats ? sizeof(Ctrl) : sizeof(CtrlHdr);
-  NWG_CUDA_TRY(cudaMemcpyAsync(ws->ctrl_host, ws->ctrl, ctrl_bytes, cudaMemcpyDeviceToHost, ws->stream));
-  NWG_CUDA_TRY(cudaStreamSynchronize(ws->stream));
+  if (stats) NWG_CUDA_TRY(cudaEventRecord(ws->ev0, ws->stream));
+  if (blk_one_fits(g->n, g->m)) {
+    // the kernel writes what the host wants into pinned memory (RMAT-10: two
+    // copies behind the traversal took longer than it)
+    rc = ws_launch_to_host(ws, root, alpha, beta, dst, parents_host != nullptr, stats != nullptr, topdown_only);
+    if (rc) return rc;
+    if (stats) NWG_CUDA_TRY(cudaEventRecord(ws->ev1, ws->stream));
+    NWG_CUDA_TRY(cudaStreamSynchronize(ws->stream));
+    if (parents_host) std::memcpy(parents_host, ws->parents_host, g->n * sizeof(uint32_t));
+  } else {
+    rc = ws_launch(ws, root, alpha, beta, dst, ws->stream, topdown_only);
+    if (rc) return rc;
+    if (stats) NWG_CUDA_TRY(cudaEventRecord(ws->ev1, ws->stream));
+    if (parents_host)
+      NWG_CUDA_TRY(cudaMemcpyAsync(parents_host, dst, g->n * sizeof(uint32_t), cudaMemcpyDeviceToHost, ws->stream));
+    const size_t ctrl_bytes = stats ? sizeof(Ctrl) : sizeof(CtrlHdr);
+    NWG_CUDA_TRY(cudaMemcpyAsync(ws->ctrl_host, ws->ctrl, ctrl_bytes, cudaMemcpyDeviceToHost, ws->stream));
+    NWG_CUDA_TRY(cudaStreamSynchronize(ws->stream));
+  }
   const Ctrl& c = *ws->ctrl_host;
   if (stats) {
     fill_stats(c, stats);

@@ -30,13 +30,29 @@ constexpr uint32_t kBlkHub   = 512;  // a vertex of more out-edges is expanded b
 constexpr uint32_t kBlkHubs  = 128;  // such vertices a step lists; further ones stay with their warp
 
 struct BlkGraph {
-  const uint64_t* off;
-  const uint32_t* col;
-  const uint64_t* in_off;
-  const uint32_t* in_col;
+  const uint64_t* off_;
+  const uint32_t* col_;
+  const uint64_t* in_off_;
+  const uint32_t* in_col_;
   const uint32_t* Z;  // in-degree-zero bitmap, or NULL: such vertices' empty lists are looked at
   uint64_t        n;
   uint64_t        m;
+  __device__ __forceinline__ uint32_t off(uint32_t v) const { return (uint32_t)__ldg(off_ + v); }
+  __device__ __forceinline__ uint32_t col(uint32_t e) const { return __ldg(col_ + e); }
+  __device__ __forceinline__ uint32_t in_off(uint32_t v) const { return (uint32_t)__ldg(in_off_ + v); }
+  __device__ __forceinline__ uint32_t in_col(uint32_t e) const { return __ldg(in_col_ + e); }
+};
+
+// The same graph copied into shared memory.
+struct BlkLocal {
+  const uint32_t *off_, *col_, *in_off_, *in_col_;
+  const uint32_t* Z;
+  uint64_t        n;
+  uint64_t        m;
+  __device__ __forceinline__ uint32_t off(uint32_t v) const { return off_[v]; }
+  __device__ __forceinline__ uint32_t col(uint32_t e) const { return col_[e]; }
+  __device__ __forceinline__ uint32_t in_off(uint32_t v) const { return in_off_[v]; }
+  __device__ __forceinline__ uint32_t in_col(uint32_t e) const { return in_col_[e]; }
 };
 
 // Queue entry, written by the step that discovers the vertex: its offsets
@@ -77,6 +93,48 @@ inline size_t blk_smem_bytes(uint64_t n) {
   return blk_fixed_bytes<T>() + blk_bitmap_bytes(n) + (n <= kBlkSmemQ ? n * sizeof(BlkEnt) : 0);
 }
 
+// A graph of at most this many bytes beside its traversal's state is copied
+// into shared memory first (bytes of the copy: blk_local_bytes).
+constexpr size_t kBlkLocalMax = 220 * 1024;
+inline size_t blk_local_bytes(uint64_t n, uint64_t m, bool symmetric) {
+  const size_t one = ((n + 1 + 3) & ~3ull) * 4 + ((m + 3) & ~3ull) * 4;
+  return symmetric ? one : 2 * one;
+}
+
+// Copies g to `at` (16-byte aligned, blk_local_bytes); ends with a barrier.
+// One SM reads RMAT-10 (94 KB) in about a microsecond; a step's loads then
+// take a shared-memory access instead of an L2 one.
+template <int T>
+__device__ __forceinline__ BlkLocal blk_copy(const BlkGraph& g, unsigned char* at) {
+  const uint32_t n = (uint32_t)g.n, m = (uint32_t)g.m;
+  const bool     one = g.in_off_ == g.off_ && g.in_col_ == g.col_;
+  uint32_t*      d   = reinterpret_cast<uint32_t*>(at);
+  BlkLocal       l{d, nullptr, nullptr, nullptr, g.Z, g.n, g.m};
+  auto           csr = [&](const uint64_t* off, const uint32_t* col, uint32_t* to) -> uint32_t* {
+    uint32_t* const tc = to + ((n + 1 + 3) & ~3u);
+    for (uint32_t i = threadIdx.x; i <= n; i += T) to[i] = (uint32_t)__ldg(off + i);
+    if ((reinterpret_cast<uintptr_t>(col) & 15) == 0) {
+      for (uint32_t i = threadIdx.x; i < m / 4; i += T)
+        reinterpret_cast<uint4*>(tc)[i] = __ldg(reinterpret_cast<const uint4*>(col) + i);
+      for (uint32_t i = (m & ~3u) + threadIdx.x; i < m; i += T) tc[i] = __ldg(col + i);
+    } else {
+      for (uint32_t i = threadIdx.x; i < m; i += T) tc[i] = __ldg(col + i);
+    }
+    return tc;
+  };
+  uint32_t* const c = csr(g.off_, g.col_, d);
+  l.col_            = c;
+  l.in_off_         = d;
+  l.in_col_         = c;
+  if (!one) {
+    uint32_t* const e = c + ((m + 3) & ~3u);
+    l.in_off_         = e;
+    l.in_col_         = csr(g.in_off_, g.in_col_, e);
+  }
+  __syncthreads();
+  return l;
+}
+
 // Enough for every graph of at most nmax vertices (a graph with its queue in
 // shared memory may need more than a larger one).
 template <int T>
@@ -87,8 +145,8 @@ inline size_t blk_smem_bytes_upto(uint64_t nmax) {
 // One round of edge tests (bfs.hpp:280-289): the lane's edges u[k] -> v[k],
 // kNull = none.  A claim's winner writes the parent and appends the vertex
 // with its offsets, one counter update per warp.  All lanes call.
-template <int T>
-__device__ __forceinline__ void blk_visit(BlkSmem<T>& sm, const BlkGraph& g, const uint32_t (&u)[kBlkVisit],
+template <int T, class G>
+__device__ __forceinline__ void blk_visit(BlkSmem<T>& sm, const G& g, const uint32_t (&u)[kBlkVisit],
                                           const uint32_t (&v)[kBlkVisit], uint32_t* V, uint32_t* parents,
                                           BlkEnt* out, uint32_t& scout) {
   const unsigned lane = threadIdx.x & 31;
@@ -105,8 +163,8 @@ __device__ __forceinline__ void blk_visit(BlkSmem<T>& sm, const BlkGraph& g, con
   for (int k = 0; k < kBlkVisit; ++k) {
     lo[k] = hi[k] = 0;
     if (win & (1u << k)) {
-      lo[k] = (uint32_t)__ldg(g.off + v[k]);
-      hi[k] = (uint32_t)__ldg(g.off + v[k] + 1);
+      lo[k] = g.off(v[k]);
+      hi[k] = g.off(v[k] + 1);
     }
   }
   const uint32_t mine = __popc(win);
@@ -129,8 +187,8 @@ __device__ __forceinline__ void blk_visit(BlkSmem<T>& sm, const BlkGraph& g, con
 // to their lanes by a prefix of the degrees; no barrier between groups, so
 // warps hide each other's latency.  Vertices of more than kBlkHub out-edges
 // are listed and then expanded by all threads.  Adds to sm.cnt, sm.scout.
-template <int T>
-__device__ __forceinline__ void blk_push(BlkSmem<T>& sm, const BlkGraph& g, const BlkEnt* q, uint32_t b, uint32_t e,
+template <int T, class G>
+__device__ __forceinline__ void blk_push(BlkSmem<T>& sm, const G& g, const BlkEnt* q, uint32_t b, uint32_t e,
                                          BlkEnt* out, uint32_t* V, uint32_t* parents) {
   const unsigned lane  = threadIdx.x & 31, wib = threadIdx.x >> 5;
   auto&          grp   = sm.grp[wib];
@@ -167,7 +225,7 @@ __device__ __forceinline__ void blk_push(BlkSmem<T>& sm, const BlkGraph& g, cons
           for (int s = 16; s >= 1; s >>= 1)
             if (grp.pre[o + s] <= i) o += s;
           u[k] = grp.u[o];
-          v[k] = __ldg(g.col + (grp.base[o] + i));
+          v[k] = g.col(grp.base[o] + i);
         }
       }
       blk_visit<T>(sm, g, u, v, V, parents, out, scout);
@@ -184,7 +242,7 @@ __device__ __forceinline__ void blk_push(BlkSmem<T>& sm, const BlkGraph& g, cons
       for (int k = 0; k < kBlkVisit; ++k) {
         const uint32_t i = e0 + k * T + lane;
         u[k]             = x.v;
-        v[k]             = i < x.deg ? __ldg(g.col + (x.lo + i)) : kNull;
+        v[k]             = i < x.deg ? g.col(x.lo + i) : kNull;
       }
       blk_visit<T>(sm, g, u, v, V, parents, out, scout);
     }
@@ -198,8 +256,8 @@ __device__ __forceinline__ void blk_push(BlkSmem<T>& sm, const BlkGraph& g, cons
 // vertices and streams them through its lanes; each lane has the next
 // candidate's offsets loading and tests kBuProbe in-edges per round.  Lists longer than kBuLane go to the warp.  V is only
 // read.  Adds the discoveries to sm.cnt.
-template <int T>
-__device__ __forceinline__ void blk_pull(BlkSmem<T>& sm, const BlkGraph& g, const uint32_t* V, const uint32_t* front,
+template <int T, class G>
+__device__ __forceinline__ void blk_pull(BlkSmem<T>& sm, const G& g, const uint32_t* V, const uint32_t* front,
                                          uint32_t* N, uint32_t* parents, uint32_t nwords) {
   const unsigned  lane    = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const unsigned  lt_mask = (1u << lane) - 1u;
@@ -226,14 +284,14 @@ __device__ __forceinline__ void blk_pull(BlkSmem<T>& sm, const BlkGraph& g, cons
     bool     cv = lane < total, nv = false;
     if (cv) {
       cu   = vbase + cand[lane];
-      cb = ce = (uint32_t)__ldg(g.in_off + cu);
-      cend    = (uint32_t)__ldg(g.in_off + cu + 1);
+      cb = ce = g.in_off(cu);
+      cend    = g.in_off(cu + 1);
     }
     uint32_t ptr = min(total, 32u);  // next unassigned list entry (warp-uniform)
     if (ptr + lane < total) {
       nu   = vbase + cand[ptr + lane];
-      nb   = (uint32_t)__ldg(g.in_off + nu);
-      nend = (uint32_t)__ldg(g.in_off + nu + 1);
+      nb   = g.in_off(nu);
+      nend = g.in_off(nu + 1);
       nv   = true;
     }
     ptr = min(total, ptr + 32u);
@@ -243,7 +301,7 @@ __device__ __forceinline__ void blk_pull(BlkSmem<T>& sm, const BlkGraph& g, cons
       if (cv) {
         uint32_t nbv[kBuProbe];
 #pragma unroll
-        for (int k = 0; k < kBuProbe; ++k) nbv[k] = ce + k < cend ? __ldg(g.in_col + (ce + k)) : kNull;
+        for (int k = 0; k < kBuProbe; ++k) nbv[k] = ce + k < cend ? g.in_col(ce + k) : kNull;
 #pragma unroll
         for (int k = kBuProbe - 1; k >= 0; --k)  // the first hit in row order stays
           if (nbv[k] != kNull && ((front[nbv[k] >> 5] >> (nbv[k] & 31)) & 1u)) {
@@ -269,7 +327,7 @@ __device__ __forceinline__ void blk_pull(BlkSmem<T>& sm, const BlkGraph& g, cons
           uint32_t       x = 0;
           bool           h = false;
           if (i < en) {
-            x = __ldg(g.in_col + i);
+            x = g.in_col(i);
             h = (front[x >> 5] >> (x & 31)) & 1u;
           }
           const unsigned hm = __ballot_sync(kFullMask, h);
@@ -302,8 +360,8 @@ __device__ __forceinline__ void blk_pull(BlkSmem<T>& sm, const BlkGraph& g, cons
         const uint32_t at   = ptr + __popc(need & lt_mask);
         if (!nv && at < total) {
           nu   = vbase + cand[at];
-          nb   = (uint32_t)__ldg(g.in_off + nu);
-          nend = (uint32_t)__ldg(g.in_off + nu + 1);
+          nb   = g.in_off(nu);
+          nend = g.in_off(nu + 1);
           nv   = true;
         }
         ptr = min(total, ptr + (uint32_t)__popc(need));
@@ -318,8 +376,8 @@ __device__ __forceinline__ void blk_pull(BlkSmem<T>& sm, const BlkGraph& g, cons
 }
 
 // The set bits of F as queue entries (bfs.hpp:235-239).
-template <int T>
-__device__ __forceinline__ void blk_b2q(BlkSmem<T>& sm, const BlkGraph& g, const uint32_t* F, uint32_t nwords,
+template <int T, class G>
+__device__ __forceinline__ void blk_b2q(BlkSmem<T>& sm, const G& g, const uint32_t* F, uint32_t nwords,
                                         BlkEnt* out) {
   const unsigned lane = threadIdx.x & 31;
   for (uint32_t w0 = threadIdx.x & ~31u; w0 < nwords; w0 += T) {
@@ -331,8 +389,8 @@ __device__ __forceinline__ void blk_b2q(BlkSmem<T>& sm, const BlkGraph& g, const
     slot = __shfl_sync(kFullMask, slot, 31) + inc - __popc(x);
     while (x) {
       const uint32_t v  = w * 32 + (__ffs(x) - 1);
-      const uint32_t lo = (uint32_t)__ldg(g.off + v);
-      out[slot++]       = BlkEnt{v, (uint32_t)__ldg(g.off + v + 1) - lo, lo, 0u};
+      const uint32_t lo = g.off(v);
+      out[slot++]       = BlkEnt{v, g.off(v + 1) - lo, lo, 0u};
       x &= x - 1;
     }
   }
@@ -343,8 +401,8 @@ __device__ __forceinline__ void blk_b2q(BlkSmem<T>& sm, const BlkGraph& g, const
 // n <= kBlkSmemQ.  trace: control block whose per-step trace is written, or
 // NULL.  All threads return the result; a barrier must come before the
 // block's next traversal.
-template <int T>
-__device__ __forceinline__ RaggedResult block_traverse(const BlkGraph& g, uint32_t root, uint32_t alpha, uint32_t beta,
+template <int T, class G>
+__device__ __forceinline__ RaggedResult block_traverse(const G& g, uint32_t root, uint32_t alpha, uint32_t beta,
                                                        bool topdown_only, uint32_t* parents, BlkEnt* q,
                                                        unsigned char* smem, Ctrl* trace, uint32_t* trace_len) {
   BlkSmem<T>&    sm     = *reinterpret_cast<BlkSmem<T>*>(smem);
@@ -373,7 +431,7 @@ __device__ __forceinline__ RaggedResult block_traverse(const BlkGraph& g, uint32
     if (t0) sm.cnt = sm.scout = sm.nhub = 0;
   };
 
-  const uint32_t rlo = (uint32_t)__ldg(g.off + root), rdeg = (uint32_t)__ldg(g.off + root + 1) - rlo;
+  const uint32_t rlo = g.off(root), rdeg = g.off(root + 1) - rlo;
   for (uint32_t w = threadIdx.x; w < nwords; w += T) V[w] = w == (root >> 5) ? 1u << (root & 31) : 0u;
   // parents := null except the root (bfs.hpp:175, 180), 16 bytes at a time
   // between the row's unaligned ends

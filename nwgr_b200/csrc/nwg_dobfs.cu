@@ -44,6 +44,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cooperative_groups.h>
+#include <cstddef>
+#include <type_traits>
 
 #include "nwg_internal.cuh"
 
@@ -70,8 +72,12 @@ constexpr uint32_t kSoloCap    = 1024;
 constexpr uint32_t kSoloLevels = 256;
 constexpr uint32_t kSoloPer    = kSoloCap / kThreads;  // list entries per thread in the prefix pass
 // One-block traversals (nwg_block.cuh): threads of the block that runs a
-// single traversal and of the blocks that run many roots of a graph.
+// single traversal, of one that copies the graph to shared memory first (its
+// steps are short: 512 threads' barriers cost less than 1,024's, 92 against
+// 97 us on a 64 x 64 grid; 256 have too few lanes, 116) and of the blocks
+// that run many roots of a graph.
 constexpr int kBlkOneT   = 1024;
+constexpr int kBlkCopyT  = 512;
 constexpr int kBlkRootsT = 512;
 // A single traversal is one block's up to these sizes.  Device time of one
 // block against the whole grid (k_trav), B200: RMAT 2^10 21 / 64 us, 2^13
@@ -2183,14 +2189,31 @@ __global__ void k_widen(const uint32_t* __restrict__ src, uint64_t* __restrict__
 
 #include "nwg_block.cuh"
 
+// Results of a one-block traversal for the host: written by the kernel into
+// pinned memory, where a copy of a few kilobytes would cost more than the
+// traversal.  ctrl: the first ctrl_vecs * 16 bytes of the control block;
+// parents: n entries; either may be NULL.
+struct BlkHost {
+  uint4*    ctrl;
+  uint32_t  ctrl_vecs;
+  uint32_t* parents;
+};
+
 // One traversal by one block; leaves the control header as k_trav does.
-__global__ void __launch_bounds__(kBlkOneT)
+// kCopy: the graph goes to shared memory first (local_at bytes into it).
+template <bool kCopy, int T>
+__global__ void __launch_bounds__(T)
     k_blk_one(BlkGraph g, uint32_t root, uint32_t alpha, uint32_t beta, uint32_t topdown_only, uint32_t* parents,
-              BlkEnt* q, Ctrl* ctrl) {
+              BlkEnt* q, Ctrl* ctrl, BlkHost host, uint32_t local_at) {
   extern __shared__ __align__(16) unsigned char blk_smem[];
-  uint32_t           ntr = 0;
-  const RaggedResult r =
-      block_traverse<kBlkOneT>(g, root, alpha, beta, topdown_only != 0, parents, q, blk_smem, ctrl, &ntr);
+  uint32_t     ntr = 0;
+  RaggedResult r;
+  if constexpr (kCopy) {
+    const BlkLocal l = blk_copy<T>(g, blk_smem + local_at);
+    r = block_traverse<T>(l, root, alpha, beta, topdown_only != 0, parents, q, blk_smem, ctrl, &ntr);
+  } else {
+    r = block_traverse<T>(g, root, alpha, beta, topdown_only != 0, parents, q, blk_smem, ctrl, &ntr);
+  }
   if (threadIdx.x == 0) {
     CtrlHdr& c     = ctrl->h;
     c.parents      = parents;
@@ -2211,6 +2234,12 @@ __global__ void __launch_bounds__(kBlkOneT)
     ctrl->decides  = 0;
     ctrl->err      = 0;
   }
+  __syncthreads();  // the block's own writes, read back below
+  if (host.ctrl)
+    for (uint32_t i = threadIdx.x; i < host.ctrl_vecs; i += T)
+      host.ctrl[i] = reinterpret_cast<const uint4*>(ctrl)[i];
+  if (host.parents)
+    for (uint32_t i = threadIdx.x; i < (uint32_t)g.n; i += T) host.parents[i] = parents[i];
 }
 
 // A ragged batch's items [first, n_items), largest first: blocks take them
@@ -2407,7 +2436,10 @@ int ws_init(GraphDev* g, Workspace* ws) {
     cudaGetLastError();
     return set_error(NWG_ENOMEM, "workspace allocation failed (n=" + std::to_string(n) + ")");
   }
-  NWG_CUDA_TRY(cudaMallocHost(&ws->ctrl_host, sizeof(Ctrl)));
+  // beside the control block, a small graph's parents for the host
+  const uint64_t host_n = blk_one_fits(n, m) ? n : 0;
+  NWG_CUDA_TRY(cudaMallocHost(&ws->ctrl_host, sizeof(Ctrl) + host_n * sizeof(uint32_t)));
+  ws->parents_host = reinterpret_cast<uint32_t*>(ws->ctrl_host + 1);
   NWG_CUDA_TRY(cudaMemset(ws->ctrl, 0, sizeof(Ctrl)));
 
   DobfsParams& P = ws->params;
@@ -2538,13 +2570,41 @@ static BlkGraph blk_graph(const DobfsParams& P) { return BlkGraph{P.off, P.col, 
 bool blk_one_fits(uint64_t n, uint64_t m) { return n <= kBlkOneN && m <= kBlkOneM; }
 
 static int blk_one_launch(const BlkGraph& g, uint32_t root, int alpha, int beta, uint32_t* parents, BlkEnt* q,
-                          Ctrl* ctrl, bool topdown_only, cudaStream_t stream) {
-  const int rc = blk_prepare<k_blk_one>();
-  if (rc) return rc;
-  k_blk_one<<<1, kBlkOneT, blk_smem_bytes<kBlkOneT>(g.n), stream>>>(g, root, (uint32_t)alpha, (uint32_t)beta,
-                                                                    topdown_only ? 1u : 0u, parents, q, ctrl);
-  NWG_CUDA_TRY(cudaGetLastError());
-  return NWG_OK;
+                          Ctrl* ctrl, bool topdown_only, const BlkHost& host, cudaStream_t stream) {
+  const bool   one   = g.in_off_ == g.off_ && g.in_col_ == g.col_;
+  const size_t local = blk_local_bytes(g.n, g.m, one);
+  auto launch = [&](auto copy_, auto threads_) -> int {
+    constexpr bool copy = decltype(copy_)::value;
+    constexpr int  T    = decltype(threads_)::value;
+    const size_t   state = (blk_smem_bytes<T>(g.n) + 15) & ~size_t(15);
+    const int      rc    = blk_prepare<k_blk_one<copy, T>>();
+    if (rc) return rc;
+    k_blk_one<copy, T><<<1, T, state + (copy ? local : 0), stream>>>(g, root, (uint32_t)alpha, (uint32_t)beta,
+                                                                     topdown_only ? 1u : 0u, parents, q, ctrl, host,
+                                                                     (uint32_t)state);
+    NWG_CUDA_TRY(cudaGetLastError());
+    return NWG_OK;
+  };
+  if (blk_smem_bytes<kBlkCopyT>(g.n) + 16 + local <= kBlkLocalMax)
+    return launch(std::true_type{}, std::integral_constant<int, kBlkCopyT>{});
+  return launch(std::false_type{}, std::integral_constant<int, kBlkOneT>{});
+}
+
+// A one-block traversal (blk_one_fits) whose control block (all of it with
+// `trace`, else its header and status) and, with parents_host, whose parents
+// the kernel writes to pinned memory: ws->ctrl_host, ws->parents_host.
+int ws_launch_to_host(Workspace* ws, uint32_t root, int alpha, int beta, uint32_t* parents, bool parents_host,
+                      bool trace, bool topdown_only) {
+  GraphDev* g = ws->g;
+  if (root >= g->n) return set_error(NWG_EINVAL, "root " + std::to_string(root) + " >= n " + std::to_string(g->n));
+  if (alpha <= 0 || beta <= 0) return set_error(NWG_EINVAL, "alpha and beta must be positive");
+  const size_t  bytes = trace ? sizeof(Ctrl) : (offsetof(Ctrl, trace_dir) + 15) & ~size_t(15);
+  const BlkHost host{reinterpret_cast<uint4*>(ws->ctrl_host), (uint32_t)(bytes / 16),
+                     parents_host ? ws->parents_host : nullptr};
+  const int rc = blk_one_launch(blk_graph(ws->params), root, alpha, beta, parents ? parents : ws->parents,
+                                reinterpret_cast<BlkEnt*>(ws->qbuf), ws->ctrl, topdown_only, host, ws->stream);
+  if (rc == NWG_OK) ws->ran = true;
+  return rc;
 }
 
 // A traversal on `stream`: one block for a small graph, else the persistent
@@ -2559,7 +2619,7 @@ int ws_launch(Workspace* ws, uint32_t root, int alpha, int beta, uint32_t* paren
   uint32_t* par    = parents ? parents : ws->parents;
   if (blk_one_fits(g->n, g->m)) {
     const int rc = blk_one_launch(blk_graph(ws->params), root, alpha, beta, par,
-                                  reinterpret_cast<BlkEnt*>(ws->qbuf), ws->ctrl, topdown_only, stream);
+                                  reinterpret_cast<BlkEnt*>(ws->qbuf), ws->ctrl, topdown_only, BlkHost{}, stream);
     if (rc) return rc;
     ws->ran = true;
     return NWG_OK;
@@ -2580,7 +2640,7 @@ int run_traversal(const DobfsParams& params, int sm_count, uint32_t root, int al
   if (blk_one_fits(P.n, P.m)) {
     BlkGraph g = blk_graph(P);
     g.Z        = nullptr;  // not built
-    return blk_one_launch(g, root, alpha, beta, parents, static_cast<BlkEnt*>(q), P.ctrl, false, stream);
+    return blk_one_launch(g, root, alpha, beta, parents, static_cast<BlkEnt*>(q), P.ctrl, false, BlkHost{}, stream);
   }
   set_density(P);
   const int rc = zero_indegree_into(P.in_off, P.n, const_cast<uint32_t*>(P.Z), sm_count, stream);

@@ -175,6 +175,7 @@ struct Workspace {
   HubRec*         hubbuf = nullptr;   // both deferred-hub record lists
   Ctrl*           ctrl = nullptr;     // device
   Ctrl*           ctrl_host = nullptr;  // pinned mirror for stats
+  uint32_t*       parents_host = nullptr;  // pinned, n entries, where one block runs a traversal (blk_one_fits)
   cudaStream_t    stream = nullptr;   // owned stream for the synchronous API
   cudaEvent_t     ev0 = nullptr, ev1 = nullptr;
   int             trav_grid = 0;     // blocks of the persistent traversal kernel (all resident)
@@ -317,6 +318,8 @@ int  ws_init(GraphDev* g, Workspace* ws);
 void ws_free(Workspace* ws);
 int  ws_launch(Workspace* ws, uint32_t root, int alpha, int beta, uint32_t* parents, cudaStream_t stream,
                bool topdown_only);
+int  ws_launch_to_host(Workspace* ws, uint32_t root, int alpha, int beta, uint32_t* parents, bool parents_host,
+                       bool trace, bool topdown_only);
 int  ws_launch_stepped(Workspace* ws, uint32_t root, int alpha, int beta, uint32_t* parents, cudaStream_t stream);
 int  run_stepped(const DobfsParams& params, int sm_count, uint32_t root, int alpha, int beta, uint32_t* parents,
                  cudaStream_t stream);
