@@ -55,6 +55,7 @@ namespace {
 constexpr int kThreads     = 256;
 constexpr int kWarps       = kThreads / 32;
 constexpr int kBuProbe     = 4;   // in-edges a lane tests per round (independent loads)
+constexpr int kBuBatch     = 4;   // candidates a lane probes at once the first time
 constexpr int kBuLane      = 32;  // in-edges a lane scans alone before the warp helps
 constexpr int kTileWords   = 16;  // bitmap words per warp tile of the bitmap->queue pass (512 vertices; <= 32)
 constexpr int kBuTileWords = 16;  // bitmap words per pull tile (512 vertices; <= 32)
@@ -786,6 +787,8 @@ __host__ __device__ __forceinline__ void set_density(DobfsParams& p) {
   p.active  = p.n > p.nzero ? p.n - p.nzero : 1;  // vertices with edges
   p.avg_deg = p.m / p.active > 1 ? p.m / p.active : 1;
 }
+// Graphs most of whose lists one probe of a pull covers.
+__host__ __device__ __forceinline__ bool sparse_graph(const DobfsParams& p) { return p.avg_deg <= kBuProbe; }
 // a > b / c for integers (c > 0) without the division: exactly a * c > b.
 __device__ __forceinline__ bool over_quotient(uint64_t a, uint64_t b, uint64_t c) {
   return __umul64hi(a, c) != 0 || a * c > b;
@@ -1435,8 +1438,9 @@ __device__ __forceinline__ uint32_t compact_tile(uint32_t bits, uint16_t* list) 
 // in-edges without a hit hands the rest of its list to the whole warp, 32
 // in-edges per step.  The first hit in row order becomes the parent, exactly
 // as the reference's sequential scan with `break`.
-__device__ __forceinline__ void bu_step(const DobfsParams& p, const StepView& sv, PullSmem& sm, uint32_t block,
-                                        uint32_t nblocks) {
+template <bool kBatch>
+__device__ __forceinline__ void bu_step_as(const DobfsParams& p, const StepView& sv, PullSmem& sm, uint32_t block,
+                                           uint32_t nblocks) {
   const uint32_t  mode    = sv.bu_mode;
   const uint32_t  bm      = sv.bm;
   uint32_t* const parents = sv.parents;
@@ -1449,6 +1453,7 @@ __device__ __forceinline__ void bu_step(const DobfsParams& p, const StepView& sv
   uint32_t* const fresh   = sm.fresh[wib];
   const uint64_t  ntiles  = (p.nwords + kBuTileWords - 1) / kBuTileWords;
   const unsigned  lt_mask = (1u << lane) - 1u;
+  constexpr int   probed  = kBatch ? kBuProbe : 0;  // in-edges the first probe has tested
   uint32_t        awake   = 0;
 
   const uint64_t  gwarp   = (uint64_t)block * kWarps + wib;
@@ -1482,24 +1487,76 @@ __device__ __forceinline__ void bu_step(const DobfsParams& p, const StepView& sv
       cm = ~(vw | fw) & ~zw;
     }
     if (lane < kBuTileWords) fresh[lane] = 0;
-    const uint32_t total = compact_tile(cm, cand);
+    uint32_t       total = compact_tile(cm, cand);
     const uint64_t vbase = t * kBuTileWords * 32;
+
+    // Meshes and roads, most of whose lists one probe covers: kBuBatch
+    // candidates a lane at once, straight through, and only the longer lists
+    // without a hit go to the streaming scan below.  Its rounds wait for one
+    // column and one front load each; here kBuBatch of both are in flight.
+    // Grid 4096^2's pulls of 1.0-1.4M front vertices 152-84 -> 110-71 us; from
+    // an average degree of 6 on the second look at the lists costs what this
+    // saves (uniform, degree 6 / 8 / 16: 405 / 430 / 511 us of pulls streamed,
+    // 410 / 442 / 515 this way; RMAT-24's dense pull 118 and 139).
+    uint32_t rest = kBatch ? 0u : total;  // candidates left for the streaming scan
+    for (uint32_t j = 0; j < total && kBatch; j += 32 * kBuBatch) {
+      uint32_t c[kBuBatch], x[kBuBatch][kBuProbe], hit[kBuBatch];
+      uint32_t d[kBuBatch];
+      uint64_t cb[kBuBatch];
+#pragma unroll
+      for (int q = 0; q < kBuBatch; ++q) {
+        const uint32_t i = j + q * 32 + lane;
+        c[q] = i < total ? cand[i] : 0u;
+        cb[q] = p.in_off[vbase + c[q]];  // (past the end: the tile's first vertex, not used)
+        d[q]  = (uint32_t)min(p.in_off[vbase + c[q] + 1] - cb[q], (uint64_t)(kBuProbe + 1));
+        if (i >= total) d[q] = 0;
+      }
+#pragma unroll
+      for (int q = 0; q < kBuBatch; ++q)
+#pragma unroll
+        for (int k = 0; k < kBuProbe; ++k) x[q][k] = k < d[q] ? __ldg(p.in_col + cb[q] + k) : kNull;
+#pragma unroll
+      for (int q = 0; q < kBuBatch; ++q) {
+        hit[q] = 0;
+#pragma unroll
+        for (int k = 0; k < kBuProbe; ++k)
+          if (x[q][k] != kNull && ((front[x[q][k] >> 5] >> (x[q][k] & 31)) & 1u)) hit[q] |= 1u << k;
+      }
+      __syncwarp();  // this batch's candidates are read; the list is refilled from its start
+#pragma unroll
+      for (int q = 0; q < kBuBatch; ++q) {
+        if (hit[q]) {
+          uint32_t par = x[q][kBuProbe - 1];
+#pragma unroll
+          for (int k = kBuProbe - 2; k >= 0; --k)
+            if (hit[q] & (1u << k)) par = x[q][k];  // the first hit in row order
+          parents[vbase + c[q]] = par;
+          atomicOr(&fresh[c[q] >> 5], 1u << (c[q] & 31));
+        }
+        const bool     more = !hit[q] && d[q] > kBuProbe;
+        const unsigned m    = __ballot_sync(kFullMask, more);
+        if (more) cand[rest + __popc(m & lt_mask)] = (uint16_t)c[q];
+        rest += __popc(m);
+      }
+    }
+    if (kBatch) __syncwarp();
+    total = rest;
 
     // current candidate (cu: local index, ce: next in-edge, cend, cn: edges
     // tested) and next candidate (nu, nb, nend, offsets in flight)
-    uint32_t cu = 0, nu = 0, cn = 0;
+    uint32_t cu = 0, nu = 0, cn = probed;
     uint64_t ce = 0, cend = 0, nb = 0, nend = 0;
     bool     cv = false, nv = false;
     if (lane < total) {
       cu   = cand[lane];
-      ce   = p.in_off[vbase + cu];
+      ce   = p.in_off[vbase + cu] + probed;
       cend = p.in_off[vbase + cu + 1];
       cv   = true;
     }
     uint32_t ptr = min(total, 32u);  // next unassigned list entry (warp-uniform)
     if (ptr + lane < total) {
       nu   = cand[ptr + lane];
-      nb   = p.in_off[vbase + nu];
+      nb   = p.in_off[vbase + nu] + probed;
       nend = p.in_off[vbase + nu + 1];
       nv   = true;
     }
@@ -1570,7 +1627,7 @@ __device__ __forceinline__ void bu_step(const DobfsParams& p, const StepView& sv
         cu   = nu;
         ce   = nb;
         cend = nend;
-        cn   = 0;
+        cn   = probed;
         cv   = true;
         nv   = false;
       }
@@ -1579,7 +1636,7 @@ __device__ __forceinline__ void bu_step(const DobfsParams& p, const StepView& sv
         const uint32_t rank = __popc(need & lt_mask);
         if (!nv && ptr + rank < total) {
           nu   = cand[ptr + rank];
-          nb   = p.in_off[vbase + nu];
+          nb   = p.in_off[vbase + nu] + probed;
           nend = p.in_off[vbase + nu + 1];
           nv   = true;
         }
@@ -1596,6 +1653,12 @@ __device__ __forceinline__ void bu_step(const DobfsParams& p, const StepView& sv
   }
   const uint32_t tot = block_sum(awake);
   if (threadIdx.x == 0 && tot) atomicAdd(sv.awake, (unsigned long long)tot);
+}
+
+__device__ __forceinline__ void bu_step(const DobfsParams& p, const StepView& sv, PullSmem& sm, uint32_t block,
+                                        uint32_t nblocks) {
+  if (sparse_graph(p)) bu_step_as<true>(p, sv, sm, block, nblocks);
+  else bu_step_as<false>(p, sv, sm, block, nblocks);
 }
 
 __global__ void __launch_bounds__(kThreads) k_bu(DobfsParams p) {
@@ -1958,6 +2021,9 @@ __device__ __forceinline__ void solo_run(const DobfsParams& p, CtrlHdr& c, SoloS
   if (c.action != kActNone && c.action != kActBU) solo_publish(p, c, c.cur, sm.q[a], na, sm.q[a ^ 1], sm);
 }
 
+// kSparse (sparse_graph): its pulls probe in batches.  An instance of its own:
+// the batches' registers would spill in the other graphs' steps.
+template <bool kSparse>
 __global__ void __launch_bounds__(kThreads, kTravPerSm)
     k_trav(DobfsParams p, uint32_t root, uint32_t alpha, uint32_t beta, uint32_t* parents, uint32_t topdown_only) {
   __shared__ StepShared sm;
@@ -2059,7 +2125,7 @@ __global__ void __launch_bounds__(kThreads, kTravPerSm)
     if (next == kActBU) {
       sv.in = sv.out = s_c.cur;
       sv.nS = sv.nC = 0;
-      bu_step(p, sv, sm.pull, blockIdx.x, gridDim.x);
+      bu_step_as<kSparse>(p, sv, sm.pull, blockIdx.x, gridDim.x);
     } else if (next == kActB2Q) {
       sv.in = sv.out = s_c.cur;
       sv.nS = sv.nC = 0;
@@ -2408,6 +2474,16 @@ int resident_grid(int sm_count, K kernel, int per_sm_cap) {
 
 }  // namespace
 
+// The persistent kernel for a graph, and its blocks: every one must be
+// resident (cooperative launch).
+static const void* trav_kernel(const DobfsParams& P) {
+  return sparse_graph(P) ? (const void*)k_trav<true> : (const void*)k_trav<false>;
+}
+static int trav_grid(const DobfsParams& P, int sm_count) {
+  return sparse_graph(P) ? resident_grid(sm_count, k_trav<true>, kTravPerSm)
+                         : resident_grid(sm_count, k_trav<false>, kTravPerSm);
+}
+
 int ws_init(GraphDev* g, Workspace* ws) {
   ws->g      = g;
   ws->device = g->device;
@@ -2469,8 +2545,7 @@ int ws_init(GraphDev* g, Workspace* ws) {
   set_density(P);
   P.symmetric    = g->symmetric ? 1u : 0u;
   P.ctrl         = ws->ctrl;
-  // every block of the persistent kernel must be resident (cooperative launch)
-  ws->trav_grid = resident_grid(g->sm_count, k_trav, kTravPerSm);
+  ws->trav_grid = trav_grid(P, g->sm_count);
   return NWG_OK;
 }
 
@@ -2626,7 +2701,7 @@ int ws_launch(Workspace* ws, uint32_t root, int alpha, int beta, uint32_t* paren
   }
   void*     args[] = {&ws->params, &r, &a, &b, &par, &td};
   NWG_CUDA_TRY(cudaMemsetAsync(&ws->ctrl->bar, 0, sizeof(GridBar), stream));
-  const int rc = coop_launch((const void*)k_trav, dim3(ws->trav_grid), args, stream);
+  const int rc = coop_launch(trav_kernel(ws->params), dim3(ws->trav_grid), args, stream);
   if (rc) return rc;
   ws->ran = true;
   return NWG_OK;
@@ -2648,7 +2723,7 @@ int run_traversal(const DobfsParams& params, int sm_count, uint32_t root, int al
   uint32_t r = root, a = (uint32_t)alpha, b = (uint32_t)beta, td = 0u;
   void*    args[] = {&P, &r, &a, &b, &parents, &td};
   NWG_CUDA_TRY(cudaMemsetAsync(&P.ctrl->bar, 0, sizeof(GridBar), stream));
-  return coop_launch((const void*)k_trav, dim3(resident_grid(sm_count, k_trav, kTravPerSm)), args, stream);
+  return coop_launch(trav_kernel(P), dim3(trav_grid(P, sm_count)), args, stream);
 }
 
 // Many roots of one graph, a block each.  A chunk of roots is one launch and
