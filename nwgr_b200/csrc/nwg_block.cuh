@@ -25,6 +25,7 @@ constexpr uint64_t kBlkMaxM = 1ull << 31;
 // Vertices up to which the queue is in shared memory too.
 constexpr uint32_t kBlkSmemQ = 2048;
 constexpr int      kBlkTile  = 8;    // bitmap words per warp tile of a pull, at most (256 vertices)
+constexpr int      kBlkBatch = 2;    // candidates a lane of a sparse graph's pull probes at once
 constexpr int      kBlkVisit = 4;    // edges a lane tests per round of a push
 constexpr uint32_t kBlkHub   = 512;  // a vertex of more out-edges is expanded by the whole block
 constexpr uint32_t kBlkHubs  = 128;  // such vertices a step lists; further ones stay with their warp
@@ -254,9 +255,13 @@ __device__ __forceinline__ void blk_push(BlkSmem<T>& sm, const G& g, const BlkEn
 // One pull (bfs.hpp:211-228) over `front` into the discovery bitmap N, as
 // bu_step: a warp takes tiles of tw bitmap words, compacts their unvisited
 // vertices and streams them through its lanes; each lane has the next
-// candidate's offsets loading and tests kBuProbe in-edges per round.  Lists longer than kBuLane go to the warp.  V is only
+// candidate's offsets loading and tests kBuProbe in-edges per round.  On
+// sparse graphs, most of whose lists one probe covers (kSparse), kBlkBatch
+// candidates a lane are probed straight through first and only longer lists
+// without a hit are streamed (a 512 x 512 grid 1.70 -> 1.63 ms, 1,024 mixed
+// items 2.11 -> 1.99 ms).  Lists longer than kBuLane go to the warp.  V is only
 // read.  Adds the discoveries to sm.cnt.
-template <int T, class G>
+template <int T, bool kSparse, class G>
 __device__ __forceinline__ void blk_pull(BlkSmem<T>& sm, const G& g, const uint32_t* V, const uint32_t* front,
                                          uint32_t* N, uint32_t* parents, uint32_t nwords) {
   const unsigned  lane    = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -264,8 +269,9 @@ __device__ __forceinline__ void blk_pull(BlkSmem<T>& sm, const G& g, const uint3
   uint16_t* const cand    = sm.cand[wib];
   // small graphs: fewer words per tile, so that every warp has one
   const uint32_t tw    = min((uint32_t)kBlkTile, (nwords + T / 32 - 1) / (T / 32));
-  const uint32_t tail  = (uint32_t)(g.n & 31);
-  uint32_t       awake = 0;
+  const uint32_t tail   = (uint32_t)(g.n & 31);
+  constexpr uint32_t probed = kSparse ? kBuProbe : 0;
+  uint32_t       awake  = 0;
   for (uint32_t w0 = wib * tw; w0 < nwords; w0 += (T / 32) * tw) {
     const uint32_t w  = w0 + lane;
     const bool     wv = lane < tw && w < nwords;
@@ -276,15 +282,49 @@ __device__ __forceinline__ void blk_pull(BlkSmem<T>& sm, const G& g, const uint3
       if (w == nwords - 1 && tail) cm &= (1u << tail) - 1u;
       N[w] = 0;
     }
-    const uint32_t total = compact_tile(cm, cand);
+    uint32_t       total = compact_tile(cm, cand);
     const uint32_t vbase = w0 * 32;
+    uint32_t       rest  = kSparse ? 0u : total;  // candidates left for the streaming scan
+    for (uint32_t j = 0; kSparse && j < total; j += 32 * kBlkBatch) {
+      uint32_t c[kBlkBatch], b[kBlkBatch], d[kBlkBatch], x[kBlkBatch][kBuProbe];
+#pragma unroll
+      for (int q = 0; q < kBlkBatch; ++q) {
+        const uint32_t i = j + q * 32 + lane;
+        c[q]             = vbase + (i < total ? cand[i] : 0u);
+        b[q]             = g.in_off(c[q]);
+        d[q]             = i < total ? g.in_off(c[q] + 1) - b[q] : 0u;
+      }
+#pragma unroll
+      for (int q = 0; q < kBlkBatch; ++q)
+#pragma unroll
+        for (int k = 0; k < kBuProbe; ++k) x[q][k] = k < d[q] ? g.in_col(b[q] + k) : kNull;
+      __syncwarp();  // this batch's candidates are read; the list is refilled from its start
+#pragma unroll
+      for (int q = 0; q < kBlkBatch; ++q) {
+        uint32_t par = kNull;
+#pragma unroll
+        for (int k = kBuProbe - 1; k >= 0; --k)  // the first hit in row order stays
+          if (x[q][k] != kNull && ((front[x[q][k] >> 5] >> (x[q][k] & 31)) & 1u)) par = x[q][k];
+        if (par != kNull) {
+          parents[c[q]] = par;
+          atomicOr(N + (c[q] >> 5), 1u << (c[q] & 31));
+        }
+        const bool     more = par == kNull && d[q] > kBuProbe;
+        const unsigned m    = __ballot_sync(kFullMask, more);
+        if (more) cand[rest + __popc(m & lt_mask)] = (uint16_t)(c[q] - vbase);
+        rest += __popc(m);
+      }
+    }
+    if (kSparse) __syncwarp();
+    total = rest;
     // current candidate (cu, next in-edge ce, end cend, first in-edge cb)
     // and the next one (nu; offsets in flight)
     uint32_t cu = 0, ce = 0, cend = 0, cb = 0, nu = 0, nb = 0, nend = 0;
     bool     cv = lane < total, nv = false;
     if (cv) {
       cu   = vbase + cand[lane];
-      cb = ce = g.in_off(cu);
+      cb   = g.in_off(cu);
+      ce   = cb + probed;
       cend    = g.in_off(cu + 1);
     }
     uint32_t ptr = min(total, 32u);  // next unassigned list entry (warp-uniform)
@@ -350,7 +390,8 @@ __device__ __forceinline__ void blk_pull(BlkSmem<T>& sm, const G& g, const uint3
       }
       if (!cv && nv) {
         cu   = nu;
-        cb = ce = nb;
+        cb   = nb;
+        ce   = nb + probed;
         cend    = nend;
         cv   = true;
         nv   = false;
@@ -461,7 +502,8 @@ __device__ __forceinline__ RaggedResult block_traverse(const G& g, uint32_t root
       bool     first = true;
       do {
         old = awake;
-        blk_pull<T>(sm, g, V, first ? V : F, N, parents, nwords);
+        if (g.m < (kBuProbe + 1) * g.n) blk_pull<T, true>(sm, g, V, first ? V : F, N, parents, nwords);
+        else blk_pull<T, false>(sm, g, V, first ? V : F, N, parents, nwords);
         __syncthreads();
         awake = sm.cnt;
         for (uint32_t w = threadIdx.x; w < nwords; w += T) V[w] |= N[w];
