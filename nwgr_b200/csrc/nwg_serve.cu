@@ -380,7 +380,7 @@ NWG_API int nwg_server_run_trace(nwg_server h, uint32_t count, const uint32_t* g
     }
     // open loop: query i is released at t0 + arrival_us[i] whatever the
     // server's progress; its latency runs from that scheduled time
-    const auto t0 = Clock::now() + std::chrono::microseconds(1000);
+    const auto t0 = Clock::now();
     uint32_t   i  = 0;
     while (i < count) {
       const auto due = t0 + std::chrono::duration_cast<Clock::duration>(std::chrono::duration<double, std::micro>(arrival_us[i]));
