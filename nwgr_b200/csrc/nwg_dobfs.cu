@@ -146,6 +146,14 @@ struct StepView {
   unsigned long long* awake;    // vertices a pull or a marking step discovers
 };
 
+// How a top-down step records its discoveries: in the next queue; in the
+// visited bitmap only (a marking step's claims); or not at all, every edge
+// u -> v storing u at v in the output queue's buffer (a marking step without
+// claims).
+constexpr int kQueue = 0;
+constexpr int kClaim = 1;
+constexpr int kOffer = 2;
+
 // ---------------------------------------------------------------------------
 // Appending discovered vertices to the next queue buffer `qi`.
 //
@@ -504,7 +512,7 @@ __device__ __forceinline__ void flush_block(const DobfsParams& p, const StepView
 // sets its bit in sv.mark and counts itself in `nbig`, which such a step
 // adds to the awake count; a marking top-down step (sv.mark_deg) adds its
 // out-degree to `scout` as well.  All 32 lanes must call.
-template <bool kDefer, bool kMark = false>
+template <bool kDefer, int kMark = kQueue>
 __device__ __forceinline__ void visit_batch(const DobfsParams& p, const StepView& sv, const uint32_t (&u)[kVisit],
                                             const uint32_t (&v)[kVisit], uint32_t valid, TdWarp& tw, uint32_t& wcnt,
                                             unsigned long long& scout, uint32_t& nbig) {
@@ -527,7 +535,7 @@ __device__ __forceinline__ void visit_batch(const DobfsParams& p, const StepView
 #pragma unroll
   for (int k = 0; k < kVisit; ++k)
     if ((try_mask & (1u << k)) && !(old[k] & (1u << (v[k] & 31)))) win |= 1u << k;
-  if (kMark) {
+  if (kMark == kClaim) {
 #pragma unroll
     for (int k = 0; k < kVisit; ++k)
       if (win & (1u << k)) parents[v[k]] = u[k];
@@ -549,6 +557,14 @@ __device__ __forceinline__ void visit_batch(const DobfsParams& p, const StepView
   if (wcnt > kWinBuf - 32 * kVisit) flush_winners<kDefer>(p, sv, tw, wcnt, scout, nbig);
 }
 
+// One batch of edges of an offering step.
+__device__ __forceinline__ void offer_batch(uint32_t* offer, const uint32_t (&u)[kVisit], const uint32_t (&v)[kVisit],
+                                            uint32_t valid) {
+#pragma unroll
+  for (int k = 0; k < kVisit; ++k)
+    if (valid & (1u << k)) offer[v[k]] = u[k];
+}
+
 // Largest range index whose exclusive prefix (in `excl`) is <= e.
 __device__ __forceinline__ int owner_of(const uint32_t* excl, uint32_t e) {
   int lo = 0;
@@ -565,7 +581,7 @@ __device__ __forceinline__ int owner_of(const uint32_t* excl, uint32_t e) {
 // range) per lane per batch; the heads and tails (< 4 edges each) are dealt
 // out as scalar edges, kVisit per lane per batch.  A unit's range is found by
 // binary search over the prefix in shared memory.  All 32 lanes must call.
-template <bool kDefer, bool kMark = false>
+template <bool kDefer, int kMark = kQueue>
 __device__ __forceinline__ void gather_ranges(const DobfsParams& p, const StepView& sv, uint32_t u, uint64_t lo,
                                               uint64_t hi, TdWarp& tw, uint32_t& wcnt, unsigned long long& scout,
                                               uint32_t& nbig) {
@@ -605,7 +621,8 @@ __device__ __forceinline__ void gather_ranges(const DobfsParams& p, const StepVi
       vv[3] = x.w;
       valid = 0xFu;
     }
-    visit_batch<kDefer, kMark>(p, sv, uu, vv, valid, tw, wcnt, scout, nbig);
+    if constexpr (kMark == kOffer) offer_batch(p.qs[sv.out], uu, vv, valid);
+    else visit_batch<kDefer, kMark>(p, sv, uu, vv, valid, tw, wcnt, scout, nbig);
   }
   for (uint32_t j = 0; j < stot; j += 32 * kVisit) {
     uint32_t uu[kVisit], vv[kVisit], valid = 0;
@@ -623,7 +640,8 @@ __device__ __forceinline__ void gather_ranges(const DobfsParams& p, const StepVi
         valid |= 1u << k;
       }
     }
-    visit_batch<kDefer, kMark>(p, sv, uu, vv, valid, tw, wcnt, scout, nbig);
+    if constexpr (kMark == kOffer) offer_batch(p.qs[sv.out], uu, vv, valid);
+    else visit_batch<kDefer, kMark>(p, sv, uu, vv, valid, tw, wcnt, scout, nbig);
   }
   __syncwarp();
 }
@@ -859,9 +877,27 @@ __device__ __forceinline__ bool mark_td(const DobfsParams& p, const CtrlHdr& c, 
   return !push_cheaper(p, c.reached + wins, wins, scout);
 }
 
+// Whether a marking step offers parents instead of claiming its discoveries.
+// An offer is one scattered store per edge and two passes over n afterwards;
+// a claim reads the visited word of every edge, and of a discovery makes an
+// atomic and a store.  Both are bound by L2's scattered accesses (about 1.2e11
+// a second), so offers win while most edges make discoveries: the front is
+// not made of hubs, whose lists overlap (RMAT-24's hub step: 152 us with
+// claims, 203 with an atomic for every edge), it has at most 2.5 out-edges per
+// vertex of the graph, and at most a quarter of the graph is visited.  Uniform
+// 2^24's step over 30M edges: 458 us with claims, 405 with an atomic for every
+// edge, 340 with offers.
+__device__ __forceinline__ uint32_t mark_offers(const DobfsParams& p, const CtrlHdr& c, uint64_t front,
+                                                uint64_t front_edges) {
+  return front_edges <= 2 * p.avg_deg * front && 2 * front_edges <= 5 * p.active && front_edges >= p.n / 2 &&
+         4 * c.reached <= p.n;
+}
+
 // Starts a marking push from the queue in c.cur; it writes C[bm ^ 1] like a
 // first pull (bm = 1: C0), and its completion is a pull's.
-__device__ __forceinline__ uint32_t mark_setup(CtrlHdr& c) {
+__device__ __forceinline__ uint32_t mark_setup(const DobfsParams& p, CtrlHdr& c, uint64_t front,
+                                               uint64_t front_edges) {
+  c.mark_offer = mark_offers(p, c, front, front_edges);
   c.bu_push   = 0;
   c.acc_awake = 0;
   c.acc_scout = 0;
@@ -871,7 +907,9 @@ __device__ __forceinline__ uint32_t mark_setup(CtrlHdr& c) {
 }
 
 // Starts a marking top-down step from the queue in c.cur (writes C0).
-__device__ __forceinline__ uint32_t mark_td_setup(CtrlHdr& c) {
+__device__ __forceinline__ uint32_t mark_td_setup(const DobfsParams& p, CtrlHdr& c, uint64_t front,
+                                                  uint64_t front_edges) {
+  c.mark_offer = mark_offers(p, c, front, front_edges);
   c.acc_awake = 0;
   c.acc_scout = 0;
   c.bm        = 1;
@@ -916,7 +954,7 @@ __device__ uint32_t decide_on(const DobfsParams& p, CtrlHdr& c, bool writer, int
           c.old_awake   = awake;                           // bfs.hpp:206
           c.awake_count = awake;
           if (pull_as_push(p, c, awake, c.acc_scout)) {
-            next = mark_push(p, c, awake, c.acc_scout) ? mark_setup(c) : td_kernel_setup(c);
+            next = mark_push(p, c, awake, c.acc_scout) ? mark_setup(p, c, awake, c.acc_scout) : td_kernel_setup(c);
           } else {  // a pull over V, which holds every visited vertex
             c.bu_push   = 0;
             c.acc_awake = 0;
@@ -1029,7 +1067,7 @@ __device__ uint32_t decide_on(const DobfsParams& p, CtrlHdr& c, bool writer, int
       c.old_awake   = nq;
       if (pull_as_push(p, c, nq, c.scout_count)) {  // scout_count: the frontier's out-edges
         if (mark_push(p, c, nq, c.scout_count)) {
-          next = mark_setup(c);
+          next = mark_setup(p, c, nq, c.scout_count);
         } else {
           c.bu_push = 1;
           next      = td_kernel_setup(c);
@@ -1043,7 +1081,7 @@ __device__ uint32_t decide_on(const DobfsParams& p, CtrlHdr& c, bool writer, int
     } else {
       c.edges_to_check -= c.scout_count;  // bfs.hpp:243
       next = td_kernel_setup(c);
-      if (mark_td(p, c, nq, c.scout_count)) next = mark_td_setup(c);
+      if (mark_td(p, c, nq, c.scout_count)) next = mark_td_setup(p, c, nq, c.scout_count);
     }
   }
   if (!done && ++c.steps > c.max_steps) {
@@ -1097,7 +1135,7 @@ __global__ void k_decide(DobfsParams p) {
 // hubs spread over the grid), then the small-degree queue; both go through
 // gather_ranges, a group of entries per warp.  The group size of chunk
 // entries shrinks when there are few so every warp gets work.
-template <bool kDefer, bool kMark = false>
+template <bool kDefer, int kMark = kQueue>
 __device__ __forceinline__ void td_step(const DobfsParams& p, const StepView& sv, TdWarp* tws, uint32_t block,
                                         uint32_t nblocks) {
   const uint32_t     cur     = sv.in;
@@ -1145,7 +1183,7 @@ __device__ __forceinline__ void td_step(const DobfsParams& p, const StepView& sv
     }
     gather_ranges<kDefer, kMark>(p, sv, u, lo, hi, tw, wcnt, scout, nbig);
   }
-  if (kMark) return;
+  if (kMark != kQueue) return;
   if (flush_light<kDefer>(p, sv, tws, wcnt, (scout | nbig) != 0)) return;
   flush_block<kDefer>(p, sv, tws, wcnt, scout, nbig, true);
 
@@ -1203,6 +1241,55 @@ __device__ __noinline__ void mark_collect(const uint32_t* V, uint32_t* mark, uin
         for (int k = 0; k < 8; ++k)
           if ((y >> k) & 1u) scout += off[v0 + k + 1] - off[v0 + k];
       }
+    }
+  }
+  const unsigned long long nf = block_sum(found);
+  __syncthreads();
+  const unsigned long long ns = block_sum(scout);
+  if (threadIdx.x == 0) {
+    if (nf) atomicAdd(awake_out, nf);
+    if (ns) atomicAdd(scout_out, ns);
+  }
+}
+
+// The discoveries of an offering step: the unvisited vertices that were
+// offered a parent take it, in vertex order; V and `mark` get their bits, the
+// counters their count and out-degree sum as in mark_collect.
+__device__ __noinline__ void offer_collect(uint32_t* V, uint32_t* mark, const uint32_t* offer, uint32_t* parents,
+                                           uint64_t n, const uint16_t* deg16, const uint64_t* off, bool deg,
+                                           unsigned long long* awake_out, unsigned long long* scout_out) {
+  const unsigned     lane   = threadIdx.x & 31;
+  const uint64_t     warp   = (uint64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
+  const uint64_t     nwarp  = (uint64_t)gridDim.x * kWarps;
+  const uint64_t     nwords = (n + 31) / 32;
+  unsigned long long found = 0, scout = 0;
+  for (uint64_t w0 = warp * 8; w0 < nwords; w0 += nwarp * 8) {  // 8 words: a vertex of each per lane
+    const uint32_t old = lane < 8 && w0 + lane < nwords ? V[w0 + lane] : ~0u;
+    uint32_t       t[8], x = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint64_t v = (w0 + j) * 32 + lane;
+      t[j]             = v < n ? offer[v] : kNull;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint64_t v    = (w0 + j) * 32 + lane;
+      const uint32_t seen = __shfl_sync(kFullMask, old, j);  // by every lane, before the test
+      const bool     hit  = t[j] != kNull && !((seen >> lane) & 1u);
+      if (hit) {
+        parents[v] = t[j];
+        ++found;
+        if (deg) {
+          const uint32_t d = deg16 ? (uint32_t)__ldg(deg16 + v) : 0xFFFFu;
+          scout += d != 0xFFFFu ? (uint64_t)d : off[v + 1] - off[v];
+        }
+      }
+      const unsigned b = __ballot_sync(kFullMask, hit);
+      if (lane == j) x = b;
+    }
+    if (lane < 8 && w0 + lane < nwords) {
+      if (x) V[w0 + lane] = old | x;
+      mark[w0 + lane] = x;
     }
   }
   const unsigned long long nf = block_sum(found);
@@ -2116,9 +2203,13 @@ __global__ void __launch_bounds__(kThreads, kTravPerSm)
     const bool      marking = next == kActBUMark || next == kActTDMark;
     uint32_t* const mark    = s_c.bm ? p.C0 : p.C1;  // the discovery bitmap of a marking step
     if (marking) {
-      // it takes the visited bitmap as it is before any claim
-      for (uint64_t w = (uint64_t)blockIdx.x * kThreads + threadIdx.x; w < p.nwords; w += (uint64_t)gridDim.x * kThreads)
-        mark[w] = p.V[w];
+      const uint64_t t0 = (uint64_t)blockIdx.x * kThreads + threadIdx.x, ts = (uint64_t)gridDim.x * kThreads;
+      if (s_c.mark_offer) {  // the next queue's buffer, which a marking step does not fill, takes the offers
+        uint32_t* const offer = p.qs[s_c.cur ^ 1u];
+        for (uint64_t v = t0; v < p.n; v += ts) offer[v] = kNull;
+      } else {  // the visited bitmap as it is before any claim
+        for (uint64_t w = t0; w < p.nwords; w += ts) mark[w] = p.V[w];
+      }
       ok = trav_barrier(p, gridDim.x, s_target);
       if (!ok) break;
     }
@@ -2137,10 +2228,15 @@ __global__ void __launch_bounds__(kThreads, kTravPerSm)
       sv.nS          = min((uint64_t)(q & 0xFFFFFFFFull), p.qs_cap);
       sv.nC          = min((uint64_t)(q >> 32), p.qc_cap);
       if (marking) {
-        td_step<true, true>(p, sv, sm.td.tw, blockIdx.x, gridDim.x);
+        if (s_c.mark_offer) td_step<true, kOffer>(p, sv, sm.td.tw, blockIdx.x, gridDim.x);
+        else td_step<true, kClaim>(p, sv, sm.td.tw, blockIdx.x, gridDim.x);
         ok = trav_barrier(p, gridDim.x, s_target);
         if (!ok) break;
         StepAcc* const acc = &p.ctrl->acc[step % 3];
+        if (s_c.mark_offer)
+          offer_collect(p.V, s_c.bm ? p.C0 : p.C1, p.qs[s_c.cur ^ 1u], s_c.parents, p.n, p.deg16, p.off,
+                        s_next == kActTDMark, &acc->awake, &acc->scout);
+        else
         mark_collect(p.V, s_c.bm ? p.C0 : p.C1, p.n, p.deg16, p.off, s_next == kActTDMark, &acc->awake, &acc->scout);
       } else {
         td_step<true>(p, sv, sm.td.tw, blockIdx.x, gridDim.x);
