@@ -2829,9 +2829,9 @@ int run_traversal(const DobfsParams& params, int sm_count, uint32_t root, int al
 struct RootsPool {
   struct Lane {
     uint32_t     slots = 0;  // roots its buffers hold
-    uint32_t*    roots = nullptr;
+    BlkEnt*      q     = nullptr;  // one allocation: queues, rows, roots
     uint32_t*    rows  = nullptr;
-    BlkEnt*      q     = nullptr;
+    uint32_t*    roots = nullptr;
     cudaStream_t s     = nullptr;
   } lane[2];
 };
@@ -2841,8 +2841,6 @@ static void lane_free(RootsPool::Lane& l) {
     cudaStreamSynchronize(l.s);
     cudaStreamDestroy(l.s);
   }
-  cudaFree(l.roots);
-  cudaFree(l.rows);
   cudaFree(l.q);
   l = RootsPool::Lane{};
 }
@@ -2881,14 +2879,15 @@ int roots_run(GraphDev* g, const uint32_t* roots, uint64_t k, int alpha, int bet
     RootsPool::Lane& l = g->roots_pool->lane[j];
     if (l.slots >= chunk) continue;
     lane_free(l);
-    if (cudaMalloc(&l.roots, chunk * sizeof(uint32_t)) != cudaSuccess ||
-        cudaMalloc(&l.rows, chunk * n * sizeof(uint32_t)) != cudaSuccess ||
-        cudaMalloc(&l.q, chunk * (n <= kBlkSmemQ ? 1 : n) * sizeof(BlkEnt)) != cudaSuccess ||
+    const uint64_t nq = chunk * (n <= kBlkSmemQ ? 1 : n);
+    if (cudaMalloc(&l.q, nq * sizeof(BlkEnt) + (chunk * n + chunk) * sizeof(uint32_t)) != cudaSuccess ||
         cudaStreamCreateWithFlags(&l.s, cudaStreamNonBlocking) != cudaSuccess) {
       cudaGetLastError();
       lane_free(l);
       return set_error(NWG_ENOMEM, "buffers of a traversal over many roots (n=" + std::to_string(n) + ")");
     }
+    l.rows  = reinterpret_cast<uint32_t*>(l.q + nq);
+    l.roots = l.rows + chunk * n;
     l.slots = chunk;
   }
   const BlkGraph bg{g->off, g->col, g->in_off, g->in_col, g->Z, g->n, g->m};
