@@ -119,8 +119,7 @@ void graph_free(GraphDev* g) {
     cudaFree(g->in_off);
     cudaFree(g->in_col);
   }
-  cudaFree(g->Z);
-  cudaFree(g->deg16);
+  cudaFree(g->tables);
   delete g;
 }
 
@@ -128,12 +127,8 @@ void graph_free(GraphDev* g) {
 // place; build the in-degree-zero bitmap and the saturated out-degrees and
 // query the SM count.
 int finish_register(GraphDev* g) {
-  cudaDeviceProp prop;
-  NWG_CUDA_TRY(cudaGetDeviceProperties(&prop, g->device));
-  g->sm_count = prop.multiProcessorCount;
-  int rc      = build_zero_indegree(g, nullptr);
-  if (rc) return rc;
-  rc = build_deg16(g, nullptr);
+  NWG_CUDA_TRY(cudaDeviceGetAttribute(&g->sm_count, cudaDevAttrMultiProcessorCount, g->device));
+  const int rc = build_vertex_tables(g, nullptr);
   if (rc) return rc;
   NWG_CUDA_TRY(cudaDeviceSynchronize());
   return NWG_OK;

@@ -2990,39 +2990,34 @@ void fill_stats(const Ctrl& c, nwg_bfs_stats* s) {
   s->first_decide_ns = c.t_first_decide;
 }
 
-// Builds the in-degree-zero bitmap Z and counts the vertices without
-// in-edges (g->nzero; the bits past n are set in Z and not counted).
-// Synchronises the stream.
-int build_deg16(GraphDev* g, cudaStream_t stream) {
-  NWG_CUDA_TRY(cudaMalloc(&g->deg16, std::max<uint64_t>(g->n, 1) * sizeof(uint16_t)));
-  if (g->n) {
-    k_deg16<<<grid_for(g, 4), kThreads, 0, stream>>>(g->off, g->n, g->deg16);
-    NWG_CUDA_TRY(cudaGetLastError());
-  }
-  return NWG_OK;
-}
-
-int build_zero_indegree(GraphDev* g, cudaStream_t stream) {
+// Builds the in-degree-zero bitmap Z, its population (g->nzero; the bits
+// past n are set in Z and not counted) and the saturated out-degrees, in one
+// allocation: allocating and freeing pieces took most of a small graph's
+// registration.  Synchronises the stream.
+int build_vertex_tables(GraphDev* g, cudaStream_t stream) {
   const uint32_t nwords = (uint32_t)((g->n + 31) / 32);
-  NWG_CUDA_TRY(cudaMalloc(&g->Z, std::max<uint32_t>(nwords, 1) * sizeof(uint32_t)));
-  g->nzero = 0;
-  if (nwords) {
-    k_zero_indegree<<<grid_for(g, 4), kThreads, 0, stream>>>(g->in_off, g->n, nwords, g->Z);
-    NWG_CUDA_TRY(cudaGetLastError());
-    unsigned long long* d = nullptr;
-    NWG_CUDA_TRY(cudaMalloc(&d, sizeof(unsigned long long)));
-    unsigned long long h  = 0;
-    cudaError_t        e  = cudaMemsetAsync(d, 0, sizeof(h), stream);
-    if (e == cudaSuccess) {
-      k_popc_words<<<grid_for(g, 4), kThreads, 0, stream>>>(g->Z, nwords, d);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    cudaFree(d);
-    if (e != cudaSuccess) return cuda_error(e, "zero in-degree count");
-    g->nzero = h - ((uint64_t)nwords * 32 - g->n);
+  const uint64_t z_at   = al(sizeof(unsigned long long));
+  const uint64_t d_at   = z_at + al(std::max<uint32_t>(nwords, 1) * sizeof(uint32_t));
+  if (cudaMalloc(&g->tables, d_at + al(std::max<uint64_t>(g->n, 1) * sizeof(uint16_t))) != cudaSuccess) {
+    cudaGetLastError();
+    g->tables = nullptr;
+    return set_error(NWG_ENOMEM, "registration tables (n=" + std::to_string(g->n) + ")");
   }
+  auto* const count = reinterpret_cast<unsigned long long*>(g->tables);
+  g->Z              = reinterpret_cast<uint32_t*>(g->tables + z_at);
+  g->deg16          = reinterpret_cast<uint16_t*>(g->tables + d_at);
+  g->nzero          = 0;
+  if (!nwords) return NWG_OK;
+  const int          grid = grid_for(g, 4);
+  unsigned long long h    = 0;
+  NWG_CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(h), stream));
+  k_zero_indegree<<<grid, kThreads, 0, stream>>>(g->in_off, g->n, nwords, g->Z);
+  k_popc_words<<<grid, kThreads, 0, stream>>>(g->Z, nwords, count);
+  k_deg16<<<grid, kThreads, 0, stream>>>(g->off, g->n, g->deg16);
+  NWG_CUDA_TRY(cudaGetLastError());
+  NWG_CUDA_TRY(cudaMemcpyAsync(&h, count, sizeof(h), cudaMemcpyDeviceToHost, stream));
+  NWG_CUDA_TRY(cudaStreamSynchronize(stream));
+  g->nzero = h - ((uint64_t)nwords * 32 - g->n);
   return NWG_OK;
 }
 

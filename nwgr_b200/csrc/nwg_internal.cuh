@@ -286,6 +286,7 @@ struct GraphDev {
   uint32_t* col = nullptr;
   uint64_t* in_off = nullptr;
   uint32_t* in_col = nullptr;
+  unsigned char* tables = nullptr;  // the allocation that holds Z and deg16
   uint32_t* Z = nullptr;  // in-degree-zero bitmap
   uint16_t* deg16 = nullptr;  // out-degrees saturated at 0xFFFF (2 bytes a vertex: mostly L2-resident)
   uint64_t  nzero = 0;    // its population (vertices without in-edges)
@@ -327,8 +328,7 @@ int  run_stepped(const DobfsParams& params, int sm_count, uint32_t root, int alp
 int  zero_indegree_into(const uint64_t* in_off, uint64_t n, uint32_t* Z, int sm_count, cudaStream_t stream);
 void fill_stats(const Ctrl& c, nwg_bfs_stats* s);
 int  depth_row16(Workspace* ws, uint32_t root, uint16_t* row, cudaStream_t stream);
-int  build_zero_indegree(GraphDev* g, cudaStream_t stream);
-int  build_deg16(GraphDev* g, cudaStream_t stream);
+int  build_vertex_tables(GraphDev* g, cudaStream_t stream);
 int  component_edges(GraphDev* g, const uint32_t* parents, uint64_t* edges, uint64_t* vertices);
 int  widen_offsets(const uint32_t* src, uint64_t* dst, uint64_t count, cudaStream_t stream);
 
