@@ -253,6 +253,17 @@ def host_graph(spec):
     return h.grid(spec["width"], spec["height"], spec["shortcut_pct"], seed=GRAPH_SEED)
 
 
+def reference_or_none():
+    """The reference's library, or None and why it is not here (it is
+    compiled from the reference's sources, which may be absent)."""
+    from oracle.oracle import Reference
+
+    try:
+        return Reference(), None
+    except (FileNotFoundError, OSError) as e:
+        return None, str(e)
+
+
 def reference_roots_timed(rg, deg, roots, order):
     """Times the reference's bfs (bfs.hpp:160-311, oracle/_ref) once per
     entry of `order` (indices into roots), wall clock around each call like
@@ -277,12 +288,14 @@ def run_reference_arm(args, spec, world, rank):
     if rank != 0:
         return
     from oracle import graphgen as gg
-    from oracle.oracle import Reference
 
+    ref, why = reference_or_none()
+    if ref is None:
+        print(json.dumps({"impl": "reference", "unavailable": why}))
+        return
     off, cols = host_graph(spec)
     roots = gg.roots(off, args.roots, seed=ROOT_SEED)
     deg = off[1:] - off[:-1]
-    ref = Reference()
     rg = ref.graph(off, cols)
     threads = ref.threads()
     for step in range(args.warmup):  # one untimed traversal per warm-up step
@@ -459,13 +472,11 @@ def bench_verifier(nwg, torch, g, roots, with_cpu):
         out["roots"].append(int(r))
         out["device_ms"].append(float(res.device_ms))
         out["valid"].append(bool(res.valid))
-    if with_cpu:
-        from oracle.oracle import Reference
-
+    ref = reference_or_none()[0] if with_cpu else None
+    if ref is not None:
         off, cols = g.csr()
         nwg.bfs_device(g, int(roots[0]), par)
         host = par.cpu().numpy().view(np.uint32)
-        ref = Reference()
         rg = ref.graph(off, cols)
         t0 = time.perf_counter()
         ok = rg.verify(int(roots[0]), host)
@@ -489,11 +500,9 @@ def bench_bc(nwg, scale=22, k=64, cpu_sample=4, with_cpu=True):
         times.append(st.device_ms)
     out = {"graph": f"RMAT-{scale} ef16", "sources": int(k), "device_ms": float(np.median(times)),
            "ms_per_source": float(np.median(times)) / k, "levels": int(st.max_levels), "lanes": int(st.lanes)}
-    if with_cpu:
-        from oracle.oracle import Reference
-
+    ref = reference_or_none()[0] if with_cpu else None
+    if ref is not None:
         off, cols = g.csr()
-        ref = Reference()
         rg = ref.graph(off, cols)
         _, secs = rg.bc(src[:cpu_sample])
         rg.close()
@@ -604,12 +613,9 @@ def bench_other_graphs(nwg, torch, main_graph, hbm, with_cpu, n_roots=64, reps=3
 def cpu_baseline(off, cols, roots, n_roots, when="before the device legs"):
     """The reference's bfs.hpp on the host cores over the first n_roots roots
     (each once; all of them by default, the roots the reference arm times)."""
-    from oracle.oracle import Reference
-
-    try:
-        ref = Reference()
-    except (FileNotFoundError, OSError) as e:
-        return {"value": None, "unit": "GTEPS", "cores": 0, "kind": "reference", "sample": f"unavailable: {e}"}
+    ref, why = reference_or_none()
+    if ref is None:
+        return {"value": None, "unit": "GTEPS", "cores": 0, "kind": "reference", "sample": f"unavailable: {why}"}
     deg = off[1:] - off[:-1]
     rg = ref.graph(off, cols)
     rg.dobfs(int(roots[0]), 32, 15, 18, want_parents=False)  # warm the pool and pages
