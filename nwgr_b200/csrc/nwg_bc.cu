@@ -35,9 +35,8 @@
 //
 // Pulls and scatters read the in-CSR.  The computation itself is defined on
 // the out-graph alone, and a graph registered without an in-CSR may in fact
-// be directed, so on its first call a graph's two CSRs are compared as sets
-// of edges (a 64-bit hash sum, 0.2 ms on RMAT-20); where they differ every
-// level pushes and gathers.
+// be directed, so the graph's two CSRs are compared (csrs_transposed); where
+// they differ every level pushes and gathers.
 //
 // Work split: eight lanes per vertex; vertices of more than kBcHub edges in
 // pieces of that many, a warp each, from a list made once per graph (a
@@ -65,7 +64,7 @@ using namespace nwg;
 namespace {
 
 constexpr int      kBcThreads = 256;
-constexpr uint32_t kBcHub     = 512;  // a vertex of more edges is split into pieces of this many
+constexpr uint32_t kBcHub     = kHubPiece;  // a vertex of more edges is split into pieces of this many
 constexpr uint32_t kBcBatch   = 32;   // most forward levels enqueued before a read-back
 constexpr uint32_t kUnset     = 0xFFFFFFFFu;
 
@@ -476,66 +475,6 @@ __global__ void k_bc_reset(BcArgs a, uint32_t s) {
   if (t == 0) a.order[0] = s;
 }
 
-// splitmix64's finalizer (Steele, Lea and Flood 2014).
-__device__ __forceinline__ uint64_t bc_mix(uint64_t x) {
-  x += 0x9E3779B97F4A7C15ull;
-  x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
-  x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
-  return x ^ (x >> 31);
-}
-
-// Adds a hash of every edge (mode 0: row -> column), takes away that of every
-// reversed edge (1), or both (2): over a CSR and its transpose the sum is
-// zero, whatever the order of their rows.
-__global__ void __launch_bounds__(kBcThreads) k_bc_edge_hash(const uint64_t* __restrict__ off,
-                                                             const uint32_t* __restrict__ col, uint64_t n,
-                                                             const uint64_t* __restrict__ piece, uint64_t npiece,
-                                                             uint32_t mode, unsigned long long* sum) {
-  const unsigned     lane  = threadIdx.x & 31;
-  const uint64_t     warp  = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint64_t     nwarp = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  unsigned long long h     = 0;
-  auto edge = [&](uint64_t u, uint64_t v) {
-    if (mode != 1) h += bc_mix((u << 32) | v);
-    if (mode != 0) h -= bc_mix((v << 32) | u);
-  };
-  for (uint64_t i = warp * 4 + (lane >> 3); i < n; i += nwarp * 4) {
-    const uint64_t e = off[i], end = off[i + 1];
-    if (end - e > kBcHub) continue;
-    for (uint64_t j = e + (lane & 7); j < end; j += 8) edge(i, __ldg(col + j));
-  }
-  for (uint64_t i = warp; i < npiece; i += nwarp) {
-    const uint64_t u  = piece[i] >> 32;
-    const uint64_t b  = off[u] + (uint64_t)(uint32_t)piece[i] * kBcHub;
-    const uint64_t en = min(off[u + 1], b + kBcHub);
-    for (uint64_t j = b + lane; j < en; j += 32) edge(u, __ldg(col + j));
-  }
-  h = bc_block_sum(h);
-  if (threadIdx.x == 0) atomicAdd(sum, h);
-}
-
-// The pieces of every vertex of more than kBcHub edges.
-__global__ void k_bc_pieces(const uint64_t* __restrict__ off, uint64_t n, uint64_t* piece, uint64_t cap,
-                            unsigned long long* count) {
-  const unsigned lane  = threadIdx.x & 31;
-  const uint64_t nwarp = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < (n + 31) / 32; w += nwarp) {
-    const uint64_t v    = w * 32 + lane;
-    const uint64_t d    = v < n ? off[v + 1] - off[v] : 0;
-    unsigned       hubs = __ballot_sync(kFullMask, d > kBcHub);
-    while (hubs) {
-      const int src = __ffs(hubs) - 1;
-      hubs &= hubs - 1;
-      const uint64_t     np   = (__shfl_sync(kFullMask, d, src) + kBcHub - 1) / kBcHub;
-      unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(count, (unsigned long long)np);
-      base = __shfl_sync(kFullMask, base, 0);
-      for (uint64_t j = lane; j < np; j += 32)
-        if (base + j < cap) piece[base + j] = ((w * 32 + src) << 32) | j;
-    }
-  }
-}
-
 // Largest score (non-negative floats: their bit patterns order as integers).
 __global__ void k_bc_max(const float* bc, uint64_t n, unsigned int* maxbits) {
   unsigned int   m      = 0;
@@ -681,47 +620,11 @@ void bc_ws_free(BcWs* w) {
 
 namespace {
 
-// The hub pieces of one direction; synchronises.
-int make_pieces(const GraphDev* g, const uint64_t* off, uint64_t m, uint64_t** piece, uint64_t* count) {
-  const uint64_t cap = 2 * (m / kBcHub) + 1;  // a vertex of d > kBcHub edges has at most 2 d / kBcHub pieces
-  if (cudaMalloc(piece, (cap + 1) * 8) != cudaSuccess) {
-    cudaGetLastError();
-    return set_error(NWG_ENOMEM, "betweenness hub list allocation failed");
-  }
-  auto* const c = reinterpret_cast<unsigned long long*>(*piece + cap);
-  NWG_CUDA_TRY(cudaMemset(c, 0, 8));
-  k_bc_pieces<<<grid_bc(g, k_bc_pieces, g->n, kBcThreads), kBcThreads>>>(off, g->n, *piece, cap, c);
-  NWG_CUDA_TRY(cudaGetLastError());
-  NWG_CUDA_TRY(cudaMemcpy(count, c, 8, cudaMemcpyDeviceToHost));
-  *count = std::min<uint64_t>(*count, cap);
-  return NWG_OK;
-}
-
-// Whether the in-CSR holds the out-CSR's edges, reversed.
-int compare_csrs(const GraphDev* g, BcWs& w) {
-  const bool          one = g->in_off == g->off && g->in_col == g->col;
-  unsigned long long* d   = nullptr;
-  unsigned long long  h   = 1;
-  NWG_CUDA_TRY(cudaMalloc(&d, sizeof h));
-  const int grid = grid_bc(g, k_bc_edge_hash, std::max(g->n, g->m / 8), kBcThreads / 8);
-  cudaError_t e  = cudaMemset(d, 0, sizeof h);
-  if (e == cudaSuccess) {
-    k_bc_edge_hash<<<grid, kBcThreads>>>(g->off, g->col, g->n, w.piece[0], w.npiece[0], one ? 2u : 0u, d);
-    if (!one) k_bc_edge_hash<<<grid, kBcThreads>>>(g->in_off, g->in_col, g->n, w.piece[1], w.npiece[1], 1u, d);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) e = cudaMemcpy(&h, d, sizeof h, cudaMemcpyDeviceToHost);
-  cudaFree(d);
-  if (e != cudaSuccess) return cuda_error(e, "comparing the two CSRs");
-  w.use_in = h == 0 && g->in_m == g->m;
-  return NWG_OK;
-}
-
 // The hub pieces and the comparison, on a graph's first call.
-int prepare(const GraphDev* g, BcWs& w) {
-  int rc = make_pieces(g, g->off, g->m, &w.piece[0], &w.npiece[0]);
-  if (!rc && g->in_off != g->off) rc = make_pieces(g, g->in_off, g->in_m, &w.piece[1], &w.npiece[1]);
-  if (!rc) rc = compare_csrs(g, w);
+int prepare(GraphDev* g, BcWs& w) {
+  int rc = hub_pieces(g, g->off, g->m, nullptr, &w.piece[0], &w.npiece[0]);
+  if (!rc && g->in_off != g->off) rc = hub_pieces(g, g->in_off, g->in_m, nullptr, &w.piece[1], &w.npiece[1]);
+  if (!rc) rc = csrs_transposed(g, &w.use_in);
   if (rc) {
     for (auto*& p : w.piece) {
       cudaFree(p);

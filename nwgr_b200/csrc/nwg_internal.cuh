@@ -295,6 +295,8 @@ struct GraphDev {
   // out-degree >= 64 goes to the chunk queue: 2.0% (RMAT-24) and 2.4%
   // (uniform 2^24) faster than 32 on a B200; 512-edge chunks gained nothing
   Thresholds th{64, 256, 8};
+  std::mutex                transposed_mu;
+  int                       transposed = -1;  // the in-CSR is the out-CSR's transpose: not compared yet, no, yes
   std::mutex                mu;
   Workspace*                default_ws = nullptr;
   Workspace*                pipe_ws    = nullptr;  // second lane of nwg_bfs_roots
@@ -345,6 +347,12 @@ void roots_pool_free(struct RootsPool* p);
 int  run_traversal(const DobfsParams& params, int sm_count, uint32_t root, int alpha, int beta, uint32_t* parents,
                    void* q, cudaStream_t stream);
 int  zero_indegree_packed(RaggedDev* r);
+
+// nwg_transpose.cu
+constexpr uint32_t kHubPiece = 512;  // a vertex of more edges is split into pieces of this many
+int hub_pieces(const GraphDev* g, const uint64_t* off, uint64_t m, cudaStream_t stream, uint64_t** piece,
+               uint64_t* count);
+int csrs_transposed(GraphDev* g, bool* yes);
 
 // nwg_verify.cu, nwg_bc.cu
 void verify_ws_free(struct VerifyWs* b);

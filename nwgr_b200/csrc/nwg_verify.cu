@@ -19,7 +19,11 @@
 // The depths' BFS: a level either pushes from a queue of 64-edge pieces of
 // its vertices (so a hub is spread over the grid: with a warp per vertex the
 // hub level of RMAT-22 alone took 4.6 of 10.4 ms) or, when its out-edges are
-// many, pulls over the visited bitmap.  No unvisited vertex has an
+// many, pulls over the visited bitmap.  Depths are defined on the out-graph
+// alone, so only a graph whose in-CSR is its out-CSR's transpose pulls
+// (csrs_transposed: the traversal under test may rest on the same in-CSR); any
+// other pushes every level, from queues that hold every level's pieces.  No
+// unvisited vertex of a graph that pulls has an
 // in-neighbour of an earlier level than the last complete one (that level
 // would have visited it), so every visited in-neighbour is one level up; the
 // pull reads one copy of the bitmap and writes the other, whose difference
@@ -74,18 +78,19 @@ struct VerifyArgs {
   const uint64_t* in_off;
   const uint32_t* in_col;
   uint64_t        n, m;
+  uint32_t        use_in;  // the in-CSR is the out-CSR's transpose: levels may pull
   uint32_t*       depth;
   uint32_t*       vis[2];  // visited bitmap, two copies
   uint64_t*       q[2];    // vertex << 32 | piece
-  uint64_t        qcap;
+  uint64_t        qcap;    // room for every level's pieces unless use_in
   VerifyCounters* cnt;
 };
 
-// Pull when the level's out-edges are a good part of what is left (and not
-// a handful), or its queue entries did not fit (more than n + m / 512
-// entries: over m / 8 out-edges).
+// Pull, where the in-CSR allows it, when the level's out-edges are a good part
+// of what is left (and not a handful), or its queue entries did not fit (more
+// than n + m / 512 entries: over m / 8 out-edges).
 __device__ __forceinline__ bool v_pulls(const VerifyArgs& a, const VerifyLevel& l) {
-  return l.entries > a.qcap || (l.edges > l.unpushed / 15 && l.edges > a.n / 32);
+  return a.use_in && (l.entries > a.qcap || (l.edges > l.unpushed / 15 && l.edges > a.n / 32));
 }
 
 __global__ void k_v_init(VerifyArgs a, uint32_t source) {
@@ -433,6 +438,7 @@ namespace nwg {
 struct VerifyWs {
   std::mutex      mu;
   bool            ready   = false;
+  bool            use_in  = false;    // csrs_transposed
   uint32_t*       depth   = nullptr;
   uint32_t*       vis     = nullptr;  // both copies
   uint64_t*       q       = nullptr;  // both queues; the pieces of long in-lists after the traversal
@@ -462,12 +468,16 @@ void verify_ws_free(VerifyWs* b) {
 
 namespace {
 
-uint64_t queue_cap(const GraphDev* g) { return g->n + g->m / 512 + 1; }
+// Entries of a queue.  Without pulls every level has to fit: at most one
+// piece that is not full for each vertex, and m / kVPiece full ones.
+uint64_t queue_cap(const GraphDev* g, bool use_in) { return g->n + g->m / (use_in ? 512 : kVPiece) + 1; }
 
-int verify_ws_make(const GraphDev* g, VerifyWs& b) {
-  const uint64_t n = std::max<uint64_t>(g->n, 1);
+int verify_ws_make(GraphDev* g, VerifyWs& b) {
+  const uint64_t n  = std::max<uint64_t>(g->n, 1);
+  const int      rc = csrs_transposed(g, &b.use_in);
+  if (rc) return rc;
   // the pieces need m / kVHub entries plus one per list of over kVHub: at most twice that
-  const uint64_t q = std::max<uint64_t>(2 * queue_cap(g), 2 * (g->in_m / kVHub) + 2);
+  const uint64_t q = std::max<uint64_t>(2 * queue_cap(g, b.use_in), 2 * (g->in_m / kVHub) + 2);
   if ((!b.depth && cudaMalloc(&b.depth, n * 4) != cudaSuccess) ||
       (!b.vis && cudaMalloc(&b.vis, 2 * ((n + 31) / 32) * 4) != cudaSuccess) ||
       (!b.q && cudaMalloc(&b.q, q * 8) != cudaSuccess) ||
@@ -502,12 +512,13 @@ int verify_on(GraphDev* g, VerifyWs& b, uint32_t source, const uint32_t* parents
   a.in_col = g->in_col;
   a.n      = n;
   a.m      = g->m;
+  a.use_in = b.use_in ? 1u : 0u;
   a.depth  = b.depth;
   a.vis[0] = b.vis;
   a.vis[1] = b.vis + (n + 31) / 32;
   a.q[0]   = b.q;
-  a.q[1]   = b.q + queue_cap(g);
-  a.qcap   = queue_cap(g);
+  a.qcap   = queue_cap(g, b.use_in);
+  a.q[1]   = b.q + a.qcap;
   a.cnt    = b.cnt;
   NWG_CUDA_TRY(cudaEventRecord(b.ev0, b.s));
   const uint32_t* par = parents_dev;
