@@ -64,7 +64,7 @@ using namespace nwg;
 namespace {
 
 constexpr int      kBcThreads = 256;
-constexpr uint32_t kBcHub     = kHubPiece;  // a vertex of more edges is split into pieces of this many
+constexpr uint32_t kBcHub     = 512;  // a vertex of more edges is split into pieces of this many
 constexpr uint32_t kBcBatch   = 32;   // most forward levels enqueued before a read-back
 constexpr uint32_t kUnset     = 0xFFFFFFFFu;
 
@@ -496,6 +496,28 @@ __global__ void k_bc_reset(BcArgs a, uint32_t s) {
   if (t == 0) a.order[0] = s;
 }
 
+// The pieces of every vertex of more than kBcHub edges.
+__global__ void k_bc_pieces(const uint64_t* __restrict__ off, uint64_t n, uint64_t* piece, uint64_t cap,
+                            unsigned long long* count) {
+  const unsigned lane  = threadIdx.x & 31;
+  const uint64_t nwarp = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < (n + 31) / 32; w += nwarp) {
+    const uint64_t v    = w * 32 + lane;
+    const uint64_t d    = v < n ? off[v + 1] - off[v] : 0;
+    unsigned       hubs = __ballot_sync(kFullMask, d > kBcHub);
+    while (hubs) {
+      const int src = __ffs(hubs) - 1;
+      hubs &= hubs - 1;
+      const uint64_t     np   = (__shfl_sync(kFullMask, d, src) + kBcHub - 1) / kBcHub;
+      unsigned long long base = 0;
+      if (lane == 0) base = atomicAdd(count, (unsigned long long)np);
+      base = __shfl_sync(kFullMask, base, 0);
+      for (uint64_t j = lane; j < np; j += 32)
+        if (base + j < cap) piece[base + j] = ((w * 32 + src) << 32) | j;
+    }
+  }
+}
+
 // Largest score (non-negative floats: their bit patterns order as integers).
 __global__ void k_bc_max(const float* bc, uint64_t n, unsigned int* maxbits) {
   unsigned int   m      = 0;
@@ -641,11 +663,27 @@ void bc_ws_free(BcWs* w) {
 
 namespace {
 
+// The hub pieces of one direction; synchronises.
+int make_pieces(const GraphDev* g, const uint64_t* off, uint64_t m, uint64_t** piece, uint64_t* count) {
+  const uint64_t cap = 2 * (m / kBcHub) + 1;  // a vertex of d > kBcHub edges has at most 2 d / kBcHub pieces
+  if (cudaMalloc(piece, (cap + 1) * 8) != cudaSuccess) {
+    cudaGetLastError();
+    return set_error(NWG_ENOMEM, "betweenness hub list allocation failed");
+  }
+  auto* const c = reinterpret_cast<unsigned long long*>(*piece + cap);
+  NWG_CUDA_TRY(cudaMemset(c, 0, 8));
+  k_bc_pieces<<<grid_bc(g, k_bc_pieces, g->n, kBcThreads), kBcThreads>>>(off, g->n, *piece, cap, c);
+  NWG_CUDA_TRY(cudaGetLastError());
+  NWG_CUDA_TRY(cudaMemcpy(count, c, 8, cudaMemcpyDeviceToHost));
+  *count = std::min<uint64_t>(*count, cap);
+  return NWG_OK;
+}
+
 // The hub pieces and the comparison, on a graph's first call.
 int prepare(GraphDev* g, BcWs& w) {
-  int rc = hub_pieces(g, g->off, g->m, nullptr, &w.piece[0], &w.npiece[0]);
-  if (!rc && g->in_off != g->off) rc = hub_pieces(g, g->in_off, g->in_m, nullptr, &w.piece[1], &w.npiece[1]);
-  if (!rc) rc = csrs_transposed(g, &w.use_in);
+  int rc = make_pieces(g, g->off, g->m, &w.piece[0], &w.npiece[0]);
+  if (!rc && g->in_off != g->off) rc = make_pieces(g, g->in_off, g->in_m, &w.piece[1], &w.npiece[1]);
+  if (!rc) rc = csrs_transposed(g, nullptr, &w.use_in);
   if (rc) {
     for (auto*& p : w.piece) {
       cudaFree(p);

@@ -286,7 +286,7 @@ struct GraphDev {
   uint32_t* col = nullptr;
   uint64_t* in_off = nullptr;
   uint32_t* in_col = nullptr;
-  unsigned char* tables = nullptr;  // the allocation that holds Z and deg16
+  unsigned char* tables = nullptr;  // the allocation that holds Z and deg16, behind a 64-bit word for sums
   uint32_t* Z = nullptr;  // in-degree-zero bitmap
   uint16_t* deg16 = nullptr;  // out-degrees saturated at 0xFFFF (2 bytes a vertex: mostly L2-resident)
   uint64_t  nzero = 0;    // its population (vertices without in-edges)
@@ -349,10 +349,7 @@ int  run_traversal(const DobfsParams& params, int sm_count, uint32_t root, int a
 int  zero_indegree_packed(RaggedDev* r);
 
 // nwg_transpose.cu
-constexpr uint32_t kHubPiece = 512;  // a vertex of more edges is split into pieces of this many
-int hub_pieces(const GraphDev* g, const uint64_t* off, uint64_t m, cudaStream_t stream, uint64_t** piece,
-               uint64_t* count);
-int csrs_transposed(GraphDev* g, bool* yes);
+int csrs_transposed(GraphDev* g, cudaStream_t stream, bool* yes);
 
 // nwg_verify.cu, nwg_bc.cu
 void verify_ws_free(struct VerifyWs* b);

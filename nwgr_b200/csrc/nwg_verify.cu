@@ -473,8 +473,9 @@ namespace {
 uint64_t queue_cap(const GraphDev* g, bool use_in) { return g->n + g->m / (use_in ? 512 : kVPiece) + 1; }
 
 int verify_ws_make(GraphDev* g, VerifyWs& b) {
-  const uint64_t n  = std::max<uint64_t>(g->n, 1);
-  const int      rc = csrs_transposed(g, &b.use_in);
+  const uint64_t n = std::max<uint64_t>(g->n, 1);
+  if (!b.s) NWG_CUDA_TRY(cudaStreamCreateWithFlags(&b.s, cudaStreamNonBlocking));
+  const int rc = csrs_transposed(g, b.s, &b.use_in);
   if (rc) return rc;
   // the pieces need m / kVHub entries plus one per list of over kVHub: at most twice that
   const uint64_t q = std::max<uint64_t>(2 * queue_cap(g, b.use_in), 2 * (g->in_m / kVHub) + 2);
@@ -486,7 +487,6 @@ int verify_ws_make(GraphDev* g, VerifyWs& b) {
     cudaGetLastError();
     return set_error(NWG_ENOMEM, "verifier allocation failed (n=" + std::to_string(g->n) + ")");
   }
-  if (!b.s) NWG_CUDA_TRY(cudaStreamCreateWithFlags(&b.s, cudaStreamNonBlocking));
   if (!b.ev0) NWG_CUDA_TRY(cudaEventCreate(&b.ev0));
   if (!b.ev1) NWG_CUDA_TRY(cudaEventCreate(&b.ev1));
   b.ready = true;
