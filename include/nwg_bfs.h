@@ -395,9 +395,8 @@ int nwg_graph_write_nwbin(nwg_graph g, const char* path);
  * for a parent array in host OR device memory (exactly one non-NULL).  Depths
  * come from a BFS over the out-graph written only for this check: it reads the
  * in-CSR to find them only where that is the out-CSR's transpose, which the
- * first call on a graph compares.  Its state (about 20 n + m / 32 bytes, m / 4
- * where the comparison fails) is kept with the graph; calls on one graph take
- * turns.  valid = 1 when the reference verifier would return true; otherwise first_bad is the
+ * first call on a graph compares.  Its state (about 8 n + m / 32 bytes, and
+ * 4 n for host parents) is kept with the graph; calls on one graph take turns.  valid = 1 when the reference verifier would return true; otherwise first_bad is the
  * lowest failing vertex (the one the reference stops at) and reason the
  * reference's failure: 1 source wrong, 2 wrong depths, 3 no edge from the
  * parent, 4 reachability mismatch.  Synchronous. */

@@ -96,6 +96,20 @@ int dev_alloc(T** p, uint64_t count) {
   return NWG_OK;
 }
 
+// The pinned slots: one block, made when first used and kept for the life of
+// the process, as allocating pinned memory takes milliseconds.
+struct PinnedPool {
+  static constexpr int kSlots = 32;
+  std::mutex           mu;
+  bool                 tried = false;
+  unsigned char*       base  = nullptr;
+  uint32_t             taken = 0;
+};
+PinnedPool& pinned_pool() {
+  static PinnedPool* p = new PinnedPool();  // outlives every caller
+  return *p;
+}
+
 void graph_free(GraphDev* g) {
   if (!g) return;
   DeviceGuard dg(g->device);
@@ -386,6 +400,39 @@ int set_error(int code, const std::string& msg) {
 int cuda_error(cudaError_t e, const char* what) {
   g_last_error = std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
   return e == cudaErrorMemoryAllocation ? NWG_ENOMEM : NWG_ECUDA;
+}
+
+PinnedSlot::PinnedSlot() : p_(nullptr), index_(-1) {
+  PinnedPool& pool = pinned_pool();
+  {
+    std::lock_guard<std::mutex> lk(pool.mu);
+    if (!pool.tried) {
+      pool.tried = true;
+      void* base = nullptr;
+      if (cudaHostAlloc(&base, PinnedPool::kSlots * kBytes, cudaHostAllocPortable) == cudaSuccess)
+        pool.base = static_cast<unsigned char*>(base);
+      else
+        cudaGetLastError();
+    }
+    for (int i = 0; pool.base && i < PinnedPool::kSlots && index_ < 0; ++i)
+      if (!((pool.taken >> i) & 1u)) index_ = i;
+    if (index_ >= 0) {
+      pool.taken |= 1u << index_;
+      p_ = pool.base + index_ * kBytes;
+      return;
+    }
+  }
+  p_ = ::operator new(kBytes, std::align_val_t(16));
+}
+
+PinnedSlot::~PinnedSlot() {
+  if (index_ < 0) {
+    ::operator delete(p_, std::align_val_t(16));
+    return;
+  }
+  PinnedPool&                 pool = pinned_pool();
+  std::lock_guard<std::mutex> lk(pool.mu);
+  pool.taken &= ~(1u << index_);
 }
 
 }  // namespace nwg

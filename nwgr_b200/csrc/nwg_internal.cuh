@@ -348,6 +348,26 @@ int  run_traversal(const DobfsParams& params, int sm_count, uint32_t root, int a
                    void* q, cudaStream_t stream);
 int  zero_indegree_packed(RaggedDev* r);
 
+// nwg_api.cu: a piece of the process's pinned memory for a call's read-backs,
+// ordinary memory where all pieces are taken; given back at the end.
+class PinnedSlot {
+ public:
+  static constexpr size_t kBytes = 2048;
+  PinnedSlot();
+  ~PinnedSlot();
+  PinnedSlot(const PinnedSlot&)            = delete;
+  PinnedSlot& operator=(const PinnedSlot&) = delete;
+  template <class T>
+  T* as() {
+    static_assert(sizeof(T) <= kBytes && alignof(T) <= 16);
+    return static_cast<T*>(p_);
+  }
+
+ private:
+  void* p_;
+  int   index_;  // -1: ordinary memory
+};
+
 // nwg_transpose.cu
 int csrs_transposed(GraphDev* g, cudaStream_t stream, bool* yes);
 

@@ -22,8 +22,9 @@
 // many, pulls over the visited bitmap.  Depths are defined on the out-graph
 // alone, so only a graph whose in-CSR is its out-CSR's transpose pulls
 // (csrs_transposed: the traversal under test may rest on the same in-CSR); any
-// other pushes every level, from queues that hold every level's pieces.  No
-// unvisited vertex of a graph that pulls has an
+// other pushes every level.  A queue holds n / 4 + m / 512 pieces; a level that
+// does not fit is pulled, or its vertices are found by their depths and each is
+// pushed by a warp.  No unvisited vertex of a graph that pulls has an
 // in-neighbour of an earlier level than the last complete one (that level
 // would have visited it), so every visited in-neighbour is one level up; the
 // pull reads one copy of the bitmap and writes the other, whose difference
@@ -35,6 +36,7 @@
 // B200: 0.5 ms against 10.4 with a warp per frontier vertex and a lane's
 // in-edges tested one by one.
 #include <algorithm>
+#include <cstddef>
 #include <mutex>
 #include <string>
 
@@ -82,13 +84,12 @@ struct VerifyArgs {
   uint32_t*       depth;
   uint32_t*       vis[2];  // visited bitmap, two copies
   uint64_t*       q[2];    // vertex << 32 | piece
-  uint64_t        qcap;    // room for every level's pieces unless use_in
+  uint64_t        qcap;
   VerifyCounters* cnt;
 };
 
 // Pull, where the in-CSR allows it, when the level's out-edges are a good part
-// of what is left (and not a handful), or its queue entries did not fit (more
-// than n + m / 512 entries: over m / 8 out-edges).
+// of what is left (and not a handful), or its queue entries did not fit.
 __device__ __forceinline__ bool v_pulls(const VerifyArgs& a, const VerifyLevel& l) {
   return a.use_in && (l.entries > a.qcap || (l.edges > l.unpushed / 15 && l.edges > a.n / 32));
 }
@@ -175,6 +176,32 @@ __device__ __forceinline__ T v_block_sum(T x) {
   return t;
 }
 
+// Pushes four edges of the lane (targets x, kUnset = none) of a vertex at
+// `level`.  All lanes call.
+__device__ __forceinline__ void v_push(const VerifyArgs& a, uint32_t* cur, uint64_t* qo, unsigned long long* entries,
+                                       uint32_t level, const uint32_t (&x)[4], unsigned long long& verts,
+                                       unsigned long long& edges) {
+  bool won[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t bit = 1u << (x[k] & 31);
+    // a stale word only costs an atomic: bits go from 0 to 1
+    won[k] = x[k] != kUnset && !(cur[x[k] >> 5] & bit) && !(atomicOr(cur + (x[k] >> 5), bit) & bit);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (!__any_sync(kFullMask, won[k])) continue;
+    uint64_t deg = 0;
+    if (won[k]) {
+      a.depth[x[k]] = level + 1;
+      deg           = a.off[x[k] + 1] - a.off[x[k]];
+      verts += 1;
+      edges += deg;
+    }
+    v_append(a, qo, entries, won[k], x[k], deg);
+  }
+}
+
 // The step of level L (depth `level`): discoveries get depth level + 1 and
 // are counted in lv[L + 1].
 __global__ void __launch_bounds__(kVThreads) k_v_step(VerifyArgs a, uint32_t L, uint32_t q, uint32_t level) {
@@ -244,7 +271,7 @@ __global__ void __launch_bounds__(kVThreads) k_v_step(VerifyArgs a, uint32_t L, 
       if (lane == 0) next[w] = seen | fresh;
     }
   } else {
-    const uint64_t  count = min(l.entries, (unsigned long long)a.qcap);
+    const uint64_t  count = l.entries > a.qcap ? 0 : l.entries;  // more: k_v_scan's
     const uint64_t* qi    = a.q[q];
     uint64_t* const qo    = a.q[q ^ 1];
     for (uint64_t i0 = warp * 4; i0 < count; i0 += nwarp * 4) {  // four entries per warp, eight lanes each
@@ -261,26 +288,40 @@ __global__ void __launch_bounds__(kVThreads) k_v_step(VerifyArgs a, uint32_t L, 
         uint32_t x[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) x[k] = e + 8 * k < end ? __ldg(a.col + e + 8 * k) : kUnset;
-        bool won[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint32_t bit = 1u << (x[k] & 31);
-          // a stale word only costs an atomic: bits go from 0 to 1
-          won[k] = x[k] != kUnset && !(cur[x[k] >> 5] & bit) && !(atomicOr(cur + (x[k] >> 5), bit) & bit);
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (!__any_sync(kFullMask, won[k])) continue;
-          uint64_t deg = 0;
-          if (won[k]) {
-            a.depth[x[k]] = level + 1;
-            deg           = a.off[x[k] + 1] - a.off[x[k]];
-            verts += 1;
-            edges += deg;
-          }
-          v_append(a, qo, &nl.entries, won[k], x[k], deg);
-        }
+        v_push(a, cur, qo, &nl.entries, level, x, verts, edges);
         e += 32;
+      }
+    }
+  }
+  const unsigned long long vs = v_block_sum(verts), es = v_block_sum(edges);
+  if (threadIdx.x == 0 && vs) {
+    atomicAdd(&nl.verts, vs);
+    atomicAdd(&nl.edges, es);
+  }
+}
+
+// The pushes of level L where its pieces did not fit the queue, on graphs that
+// may not pull: the level's vertices are found by their depths, a warp each.
+__global__ void __launch_bounds__(kVThreads) k_v_scan(VerifyArgs a, uint32_t L, uint32_t q, uint32_t level) {
+  const VerifyLevel l = a.cnt->lv[L];
+  if (l.verts == 0 || l.entries <= a.qcap) return;
+  VerifyLevel&       nl    = a.cnt->lv[L + 1];
+  uint32_t* const    cur   = a.vis[0];  // only pulls change copies
+  const unsigned     lane  = threadIdx.x & 31;
+  const uint64_t     nwarp = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  unsigned long long verts = 0, edges = 0;
+  for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32 < a.n; w += nwarp) {
+    const uint64_t u    = w * 32 + lane;
+    unsigned       pend = __ballot_sync(kFullMask, u < a.n && a.depth[u] == level);
+    while (pend) {
+      const uint64_t us = w * 32 + __ffs(pend) - 1;
+      pend &= pend - 1;
+      const uint64_t end = a.off[us + 1];
+      for (uint64_t e = a.off[us]; e < end; e += 32 * 4) {
+        uint32_t x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x[k] = e + k * 32 + lane < end ? __ldg(a.col + e + k * 32 + lane) : kUnset;
+        v_push(a, cur, a.q[q ^ 1], &nl.entries, level, x, verts, edges);
       }
     }
   }
@@ -435,16 +476,20 @@ namespace nwg {
 
 // The check's state, made on a graph's first verification and kept with it
 // (making and freeing it took 2 ms of a call); calls on one graph take turns.
+// The counters are read through a slot of the process's pinned memory: with a
+// pinned mirror of its own a first verification of a graph of 1,024 vertices
+// took 2.0-4.0 ms, 0.26 so; read into ordinary memory, a call over 40
+// levels took 4% longer.  One allocation for all arrays made a uniform graph of
+// 2^24 vertices 3% slower (12.5 ms against 12.9).
 struct VerifyWs {
   std::mutex      mu;
   bool            ready   = false;
   bool            use_in  = false;    // csrs_transposed
+  VerifyCounters* cnt     = nullptr;
   uint32_t*       depth   = nullptr;
   uint32_t*       vis     = nullptr;  // both copies
   uint64_t*       q       = nullptr;  // both queues; the pieces of long in-lists after the traversal
   uint32_t*       par     = nullptr;  // device copy of host parents, made when first needed
-  VerifyCounters* cnt     = nullptr;
-  VerifyCounters* cnt_host = nullptr;  // pinned
   cudaStream_t    s       = nullptr;
   cudaEvent_t     ev0 = nullptr, ev1 = nullptr;
 };
@@ -455,9 +500,8 @@ void verify_ws_free(VerifyWs* b) {
   cudaFree(b->depth);
   cudaFree(b->vis);
   cudaFree(b->q);
-  cudaFree(b->par);
   cudaFree(b->cnt);
-  if (b->cnt_host) cudaFreeHost(b->cnt_host);
+  cudaFree(b->par);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->s) cudaStreamDestroy(b->s);
@@ -468,22 +512,18 @@ void verify_ws_free(VerifyWs* b) {
 
 namespace {
 
-// Entries of a queue.  Without pulls every level has to fit: at most one
-// piece that is not full for each vertex, and m / kVPiece full ones.
-uint64_t queue_cap(const GraphDev* g, bool use_in) { return g->n + g->m / (use_in ? 512 : kVPiece) + 1; }
+uint64_t queue_cap(const GraphDev* g) { return g->n / 4 + g->m / 512 + 1; }
 
 int verify_ws_make(GraphDev* g, VerifyWs& b) {
-  const uint64_t n = std::max<uint64_t>(g->n, 1);
   if (!b.s) NWG_CUDA_TRY(cudaStreamCreateWithFlags(&b.s, cudaStreamNonBlocking));
   const int rc = csrs_transposed(g, b.s, &b.use_in);
   if (rc) return rc;
   // the pieces need m / kVHub entries plus one per list of over kVHub: at most twice that
-  const uint64_t q = std::max<uint64_t>(2 * queue_cap(g, b.use_in), 2 * (g->in_m / kVHub) + 2);
-  if ((!b.depth && cudaMalloc(&b.depth, n * 4) != cudaSuccess) ||
-      (!b.vis && cudaMalloc(&b.vis, 2 * ((n + 31) / 32) * 4) != cudaSuccess) ||
+  const uint64_t q = std::max<uint64_t>(2 * queue_cap(g), 2 * (g->in_m / kVHub) + 2);
+  if ((!b.depth && cudaMalloc(&b.depth, g->n * 4) != cudaSuccess) ||
+      (!b.vis && cudaMalloc(&b.vis, 2 * ((g->n + 31) / 32) * 4) != cudaSuccess) ||
       (!b.q && cudaMalloc(&b.q, q * 8) != cudaSuccess) ||
-      (!b.cnt && cudaMalloc(&b.cnt, sizeof(VerifyCounters)) != cudaSuccess) ||
-      (!b.cnt_host && cudaMallocHost(&b.cnt_host, sizeof(VerifyCounters)) != cudaSuccess)) {
+      (!b.cnt && cudaMalloc(&b.cnt, sizeof(VerifyCounters)) != cudaSuccess)) {
     cudaGetLastError();
     return set_error(NWG_ENOMEM, "verifier allocation failed (n=" + std::to_string(g->n) + ")");
   }
@@ -517,7 +557,7 @@ int verify_on(GraphDev* g, VerifyWs& b, uint32_t source, const uint32_t* parents
   a.vis[0] = b.vis;
   a.vis[1] = b.vis + (n + 31) / 32;
   a.q[0]   = b.q;
-  a.qcap   = queue_cap(g, b.use_in);
+  a.qcap   = queue_cap(g);
   a.q[1]   = b.q + a.qcap;
   a.cnt    = b.cnt;
   NWG_CUDA_TRY(cudaEventRecord(b.ev0, b.s));
@@ -531,18 +571,21 @@ int verify_on(GraphDev* g, VerifyWs& b, uint32_t source, const uint32_t* parents
   const int gw = grid_v(g, std::max(n, g->m / kVPiece), kVThreads);  // a step's grid: levels of any size
   uint32_t  base = 0;  // depth of the batch's first level, lv[0]
   uint32_t  levels = 0;
+  PinnedSlot      slot;
+  VerifyCounters& hc = *slot.as<VerifyCounters>();
   // the first read-back after eight levels (hub graphs have 5-9), then every kVBatch
   for (uint32_t done = 0, until = 8;;) {
     for (; done < until; ++done) {
       const uint32_t level = base + done;
       k_v_queue<<<gw, kVThreads, 0, b.s>>>(a, done, level & 1);
+      if (!b.use_in) k_v_scan<<<gw, kVThreads, 0, b.s>>>(a, done, level & 1, level);
       k_v_step<<<gw, kVThreads, 0, b.s>>>(a, done, level & 1, level);
     }
     NWG_CUDA_TRY(cudaGetLastError());
-    NWG_CUDA_TRY(cudaMemcpyAsync(b.cnt_host, b.cnt, sizeof(VerifyCounters), cudaMemcpyDeviceToHost, b.s));
+    NWG_CUDA_TRY(cudaMemcpyAsync(&hc, b.cnt, sizeof hc, cudaMemcpyDeviceToHost, b.s));
     NWG_CUDA_TRY(cudaStreamSynchronize(b.s));
-    if (b.cnt_host->lv[done].verts == 0) {
-      while (b.cnt_host->lv[done].verts == 0) --done;  // lv[0] holds a vertex
+    if (hc.lv[done].verts == 0) {
+      while (hc.lv[done].verts == 0) --done;  // lv[0] holds a vertex
       levels = base + done + 1;
       break;
     }
@@ -561,15 +604,14 @@ int verify_on(GraphDev* g, VerifyWs& b, uint32_t source, const uint32_t* parents
   k_v_verdicts<<<grid_v(g, g->in_m / kVHub, kVThreads), kVThreads, 0, b.s>>>(a, par, b.q, b.vis);
   NWG_CUDA_TRY(cudaGetLastError());
   NWG_CUDA_TRY(cudaEventRecord(b.ev1, b.s));
-  NWG_CUDA_TRY(cudaMemcpyAsync(b.cnt_host, b.cnt, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, b.s));
+  NWG_CUDA_TRY(cudaMemcpyAsync(&hc, b.cnt, offsetof(VerifyCounters, lv), cudaMemcpyDeviceToHost, b.s));
   NWG_CUDA_TRY(cudaStreamSynchronize(b.s));
-  const VerifyCounters& hc = *b.cnt_host;
-  nwg_verify_result     r  = {};
-  r.valid                  = hc.first == ~0ull ? 1 : 0;
-  r.reason                 = r.valid ? 0u : (uint32_t)(hc.first & 7u);
-  r.first_bad              = r.valid ? ~0ull : (hc.first >> 3);
-  r.reached                = hc.reached;
-  r.levels                 = levels;
+  nwg_verify_result r = {};
+  r.valid             = hc.first == ~0ull ? 1 : 0;
+  r.reason            = r.valid ? 0u : (uint32_t)(hc.first & 7u);
+  r.first_bad         = r.valid ? ~0ull : (hc.first >> 3);
+  r.reached           = hc.reached;
+  r.levels            = levels;
   cudaEventElapsedTime(&r.device_ms, b.ev0, b.ev1);
   *out = r;
   return NWG_OK;
