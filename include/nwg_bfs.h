@@ -357,8 +357,8 @@ int nwg_bfs_noalloc(const uint64_t* out_off, const uint32_t* out_col, const uint
  * level first, every reached vertex (the source included) adding its own;
  * scores divided by the largest when normalize != 0.  `lanes` sources run
  * at once (0 = 4, at most 16), one stream each; their state (28 n bytes a
- * lane, when that is at most 1 GB in all) is kept with the graph, and calls on
- * one graph take turns.  Scores (n floats) go to
+ * lane, when that is at most 1 GB in all) is kept with the graph, and a call
+ * that runs beside another on the same graph makes and frees its own.  Scores (n floats) go to
  * scores_host and/or scores_dev; float sums across sources, as in the
  * reference, so results agree with it within the reference verifier's
  * tolerance (1e-6 on normalized scores), not bit for bit. */
@@ -396,9 +396,10 @@ int nwg_graph_write_nwbin(nwg_graph g, const char* path);
  * come from a BFS over the out-graph written only for this check: it reads the
  * in-CSR to find them only where that is the out-CSR's transpose, which the
  * first call on a graph compares.  Its state (about 8 n + m / 32 bytes, and
- * 4 n for host parents) is kept with the graph; calls on one graph take turns.  valid = 1 when the reference verifier would return true; otherwise first_bad is the
- * lowest failing vertex (the one the reference stops at) and reason the
- * reference's failure: 1 source wrong, 2 wrong depths, 3 no edge from the
+ * 4 n for host parents) is kept with the graph; a call that runs beside another
+ * on the same graph makes and frees its own.  valid = 1 when the reference
+ * verifier would return true; otherwise first_bad is the lowest failing vertex
+ * (the one the reference stops at) and reason the reference's failure: 1 source wrong, 2 wrong depths, 3 no edge from the
  * parent, 4 reachability mismatch.  Synchronous. */
 typedef struct {
   int32_t valid;

@@ -50,7 +50,6 @@
 // sources, as in the reference.
 #include <algorithm>
 #include <atomic>
-#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -634,9 +633,9 @@ namespace nwg {
 
 // The lanes, hub pieces and score array of a graph.  Making and freeing them
 // took 14-25 ms of a call with 4 lanes on RMAT-20, so they are kept with the
-// graph (lanes up to kBcKeep bytes); calls on one graph take turns.
+// graph (lanes up to kBcKeep bytes); a call beside another on the same graph
+// makes its own.
 struct BcWs {
-  std::mutex          mu;
   std::vector<BcSlab> slabs;
   std::vector<BcSlot> slots;
   uint64_t*           piece[2]  = {nullptr, nullptr};  // out, in
@@ -866,16 +865,10 @@ NWG_API int nwg_bc(nwg_graph h, const uint32_t* sources, uint32_t k, int normali
       int d;
       ~Restore() { cudaSetDevice(d); }
     } restore{prev};
-    BcWs* w = nullptr;
-    {
-      std::lock_guard<std::mutex> lk(g->mu);
-      if (!g->bc_ws) g->bc_ws = new BcWs();
-      w = g->bc_ws;
-    }
-    std::lock_guard<std::mutex> lk(w->mu);
+    KeptState<BcWs, bc_ws_free> w(g->kept_mu, g->bc_ws);
     const int rc = bc_run(g, *w, sources, k, normalize, lanes, scores_host, scores_dev, stats);
-    // after an error a lane's dsum may not be zero
-    if (rc || w->slots.size() * BcLayout(g->n).bytes > kBcKeep) slabs_free(w->slabs, w->slots);
+    if (w->slots.size() * BcLayout(g->n).bytes > kBcKeep) slabs_free(w->slabs, w->slots);
+    if (!rc) w.keep();  // (after an error a lane's dsum may not be zero)
     return rc;
   } catch (const std::exception& ex) {
     return set_error(NWG_ENOMEM, std::string("betweenness failed: ") + ex.what());

@@ -7,6 +7,7 @@
 
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "nwg_bfs.h"
@@ -300,8 +301,9 @@ struct GraphDev {
   std::mutex                mu;
   Workspace*                default_ws = nullptr;
   Workspace*                pipe_ws    = nullptr;  // second lane of nwg_bfs_roots
-  struct VerifyWs*          verify_ws  = nullptr;  // state of nwg_verify
-  struct BcWs*              bc_ws      = nullptr;  // state of nwg_bc
+  std::mutex                kept_mu;               // guards the next two pointers
+  struct VerifyWs*          verify_ws  = nullptr;  // state of nwg_verify, NULL while a call has it
+  struct BcWs*              bc_ws      = nullptr;  // state of nwg_bc, likewise
   struct RootsPool*         roots_pool = nullptr;  // its rows and queues where blocks take the roots
   std::vector<Workspace*>   workspaces;
   std::vector<MsWorkspace*> ms_workspaces;
@@ -374,6 +376,33 @@ int csrs_transposed(GraphDev* g, cudaStream_t stream, bool* yes);
 // nwg_verify.cu, nwg_bc.cu
 void verify_ws_free(struct VerifyWs* b);
 void bc_ws_free(struct BcWs* w);
+
+// A call's state of type T: the one kept in `kept`, or a new one where there is
+// none or another call has it, so calls on one graph run side by side.  After
+// keep() it is kept again, if no other call's is; otherwise it is freed.
+template <class T, void (*Free)(T*)>
+class KeptState {
+ public:
+  KeptState(std::mutex& mu, T*& kept) : mu_(mu), kept_(kept) {
+    std::lock_guard<std::mutex> lk(mu_);
+    std::swap(s_, kept_);
+    if (!s_) s_ = new T();
+  }
+  ~KeptState() { Free(s_); }
+  KeptState(const KeptState&)            = delete;
+  KeptState& operator=(const KeptState&) = delete;
+  T& operator*() { return *s_; }
+  T* operator->() { return s_; }
+  void keep() {
+    std::lock_guard<std::mutex> lk(mu_);
+    if (!kept_) std::swap(s_, kept_);
+  }
+
+ private:
+  std::mutex& mu_;
+  T*&         kept_;
+  T*          s_ = nullptr;
+};
 
 // nwg_msbfs.cu
 int      ms_ws_init(GraphDev* g, MsWorkspace* ws);

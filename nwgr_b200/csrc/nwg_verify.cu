@@ -37,7 +37,6 @@
 // in-edges tested one by one.
 #include <algorithm>
 #include <cstddef>
-#include <mutex>
 #include <string>
 
 #include "nwg_internal.cuh"
@@ -475,14 +474,14 @@ int grid_v(const GraphDev* g, uint64_t items, uint64_t per_block) {
 namespace nwg {
 
 // The check's state, made on a graph's first verification and kept with it
-// (making and freeing it took 2 ms of a call); calls on one graph take turns.
+// (making and freeing it took 2 ms of a call); a call beside another on the
+// same graph makes its own.
 // The counters are read through a slot of the process's pinned memory: with a
 // pinned mirror of its own a first verification of a graph of 1,024 vertices
 // took 2.0-4.0 ms, 0.26 so; read into ordinary memory, a call over 40
 // levels took 4% longer.  One allocation for all arrays made a uniform graph of
 // 2^24 vertices 3% slower (12.5 ms against 12.9).
 struct VerifyWs {
-  std::mutex      mu;
   bool            ready   = false;
   bool            use_in  = false;    // csrs_transposed
   VerifyCounters* cnt     = nullptr;
@@ -619,14 +618,10 @@ int verify_on(GraphDev* g, VerifyWs& b, uint32_t source, const uint32_t* parents
 
 int verify(GraphDev* g, uint32_t source, const uint32_t* parents_host, const uint32_t* parents_dev,
            nwg_verify_result* out) {
-  VerifyWs* b = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(g->mu);
-    if (!g->verify_ws) g->verify_ws = new VerifyWs();
-    b = g->verify_ws;
-  }
-  std::lock_guard<std::mutex> lk(b->mu);
-  return verify_on(g, *b, source, parents_host, parents_dev, out);
+  KeptState<VerifyWs, verify_ws_free> b(g->kept_mu, g->verify_ws);
+  const int rc = verify_on(g, *b, source, parents_host, parents_dev, out);
+  if (!rc) b.keep();
+  return rc;
 }
 
 }  // namespace
