@@ -121,7 +121,9 @@ int nwg_bfs(nwg_graph g, uint32_t root, int alpha, int beta, uint32_t* parents_h
  * bfs(graph, gx, source, num_bins, alpha, beta) once per source.  On small
  * graphs (at most 2^19 vertices) many roots traverse side by side, one block
  * each, and their rows are copied a launch at a time (buffers of up to 128 MB
- * are kept with the graph).  Otherwise two
+ * are kept with the graph).  What this call, nwg_verify and nwg_bc keep for a
+ * next call is at most 1 GB for one of them and 2 GB in all on a device; what is
+ * past that is freed before the call returns.  Otherwise two
  * traversals are in flight: root i + 1 runs on the device while root i's
  * parents cross to the host, so with pinned host memory a call costs about
  * k copies of n * 4 bytes rather than k copies plus k traversals (pageable

@@ -3,6 +3,7 @@
 // stream-ordered BFS entry points, and per-thread error messages.  No C++
 // exception crosses this file's functions.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <exception>
 #include <new>
@@ -400,6 +401,22 @@ int set_error(int code, const std::string& msg) {
 int cuda_error(cudaError_t e, const char* what) {
   g_last_error = std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
   return e == cudaErrorMemoryAllocation ? NWG_ENOMEM : NWG_ECUDA;
+}
+
+namespace {
+constexpr int         kKeptDevices = 64;
+std::atomic<uint64_t> g_kept[kKeptDevices];
+}  // namespace
+
+bool keep_bytes(int device, uint64_t bytes) {
+  if (device < 0 || device >= kKeptDevices || bytes > kKeptState) return false;
+  if (g_kept[device].fetch_add(bytes) + bytes <= kKeptAll) return true;
+  g_kept[device].fetch_sub(bytes);
+  return false;
+}
+
+void drop_bytes(int device, uint64_t bytes) {
+  if (bytes) g_kept[device].fetch_sub(bytes);
 }
 
 PinnedSlot::PinnedSlot() : p_(nullptr), index_(-1) {

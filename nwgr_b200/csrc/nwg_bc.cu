@@ -623,19 +623,17 @@ int add_lanes(const GraphDev* g, std::vector<BcSlab>& slabs, std::vector<BcSlot>
   return NWG_OK;
 }
 
-// The most that is kept with the graph between calls (4 lanes of 2^23
-// vertices).
-constexpr uint64_t kBcKeep = 1ull << 30;
-
 }  // namespace
 
 namespace nwg {
 
 // The lanes, hub pieces and score array of a graph.  Making and freeing them
 // took 14-25 ms of a call with 4 lanes on RMAT-20, so they are kept with the
-// graph (lanes up to kBcKeep bytes); a call beside another on the same graph
-// makes its own.
+// graph (up to 1 GB: 4 lanes of 2^23 vertices); a call beside another on the
+// same graph makes its own.
 struct BcWs {
+  int                 device     = 0;
+  uint64_t            kept_bytes = 0;
   std::vector<BcSlab> slabs;
   std::vector<BcSlot> slots;
   uint64_t*           piece[2]  = {nullptr, nullptr};  // out, in
@@ -649,6 +647,7 @@ struct BcWs {
 
 void bc_ws_free(BcWs* w) {
   if (!w) return;
+  drop_bytes(w->device, w->kept_bytes);
   slabs_free(w->slabs, w->slots);
   for (auto* p : w->piece) cudaFree(p);
   cudaFree(w->bc);
@@ -867,8 +866,10 @@ NWG_API int nwg_bc(nwg_graph h, const uint32_t* sources, uint32_t k, int normali
     } restore{prev};
     KeptState<BcWs, bc_ws_free> w(g->kept_mu, g->bc_ws);
     const int rc = bc_run(g, *w, sources, k, normalize, lanes, scores_host, scores_dev, stats);
-    if (w->slots.size() * BcLayout(g->n).bytes > kBcKeep) slabs_free(w->slabs, w->slots);
-    if (!rc) w.keep();  // (after an error a lane's dsum may not be zero)
+    // (after an error a lane's dsum may not be zero)
+    if (!rc)
+      w.keep(g->device, w->slots.size() * BcLayout(g->n).bytes + (w->bc ? 4 * g->n : 0) +
+                            8 * (2 * (g->m / kBcHub) + 2) * (w->piece[1] ? 2 : 1));
     return rc;
   } catch (const std::exception& ex) {
     return set_error(NWG_ENOMEM, std::string("betweenness failed: ") + ex.what());

@@ -2827,8 +2827,11 @@ int run_traversal(const DobfsParams& params, int sm_count, uint32_t root, int al
 // queues and stream, so a chunk's rows cross to the host while the next
 // traverses.
 struct RootsPool {
+  int      device     = 0;
+  uint64_t kept_bytes = 0;
   struct Lane {
     uint32_t     slots = 0;  // roots its buffers hold
+    uint64_t     bytes = 0;
     BlkEnt*      q     = nullptr;  // one allocation: queues, rows, roots
     uint32_t*    rows  = nullptr;
     uint32_t*    roots = nullptr;
@@ -2847,6 +2850,7 @@ static void lane_free(RootsPool::Lane& l) {
 
 void roots_pool_free(RootsPool* p) {
   if (!p) return;
+  drop_bytes(p->device, p->kept_bytes);
   for (auto& l : p->lane) lane_free(l);
   delete p;
 }
@@ -2869,18 +2873,19 @@ bool roots_by_block(const GraphDev* g, uint64_t k) {
   return waves * (20.0 + 0.004 * blk_weight(g->n, g->m)) < 60.0 * (double)k;
 }
 
-int roots_run(GraphDev* g, const uint32_t* roots, uint64_t k, int alpha, int beta, uint32_t* parents_host) {
+static int roots_lanes_run(GraphDev* g, const uint32_t* roots, uint64_t k, int alpha, int beta,
+                           uint32_t* parents_host) {
   const uint64_t n  = g->n;
   const int      rc = blk_prepare<k_blk_roots>();
   if (rc) return rc;
   const uint32_t chunk = (uint32_t)std::min<uint64_t>(k, roots_slots(g));
-  if (!g->roots_pool) g->roots_pool = new RootsPool();
   for (int j = 0; j < (k > chunk ? 2 : 1); ++j) {
     RootsPool::Lane& l = g->roots_pool->lane[j];
     if (l.slots >= chunk) continue;
     lane_free(l);
     const uint64_t nq = chunk * (n <= kBlkSmemQ ? 1 : n);
-    if (cudaMalloc(&l.q, nq * sizeof(BlkEnt) + (chunk * n + chunk) * sizeof(uint32_t)) != cudaSuccess ||
+    l.bytes = nq * sizeof(BlkEnt) + (chunk * n + chunk) * sizeof(uint32_t);
+    if (cudaMalloc(&l.q, l.bytes) != cudaSuccess ||
         cudaStreamCreateWithFlags(&l.s, cudaStreamNonBlocking) != cudaSuccess) {
       cudaGetLastError();
       lane_free(l);
@@ -2910,6 +2915,22 @@ int roots_run(GraphDev* g, const uint32_t* roots, uint64_t k, int alpha, int bet
   }
   if (e != cudaSuccess) return cuda_error(e, "traversals over many roots");
   return NWG_OK;
+}
+
+// Called under g->mu.
+int roots_run(GraphDev* g, const uint32_t* roots, uint64_t k, int alpha, int beta, uint32_t* parents_host) {
+  if (!g->roots_pool) g->roots_pool = new RootsPool();
+  RootsPool& p  = *g->roots_pool;
+  const int  rc = roots_lanes_run(g, roots, k, alpha, beta, parents_host);
+  drop_bytes(p.device, p.kept_bytes);
+  p.device     = g->device;
+  p.kept_bytes = p.lane[0].bytes + p.lane[1].bytes;
+  if (rc || !keep_bytes(p.device, p.kept_bytes)) {
+    p.kept_bytes = 0;
+    roots_pool_free(g->roots_pool);
+    g->roots_pool = nullptr;
+  }
+  return rc;
 }
 
 // The level loop driven from the host: the kernels of the CUDA graph

@@ -377,9 +377,19 @@ int csrs_transposed(GraphDev* g, cudaStream_t stream, bool* yes);
 void verify_ws_free(struct VerifyWs* b);
 void bc_ws_free(struct BcWs* w);
 
+// nwg_api.cu: device memory that graphs keep between calls for the next call's
+// sake (states of nwg_verify, nwg_bc and nwg_bfs_roots), at most kKeptState of
+// one and kKeptAll of all graphs of a device.  keep_bytes says whether `bytes`
+// may be kept and counts them; drop_bytes takes them back.
+constexpr uint64_t kKeptState = 1ull << 30;
+constexpr uint64_t kKeptAll   = 2ull << 30;
+bool keep_bytes(int device, uint64_t bytes);
+void drop_bytes(int device, uint64_t bytes);
+
 // A call's state of type T: the one kept in `kept`, or a new one where there is
 // none or another call has it, so calls on one graph run side by side.  After
-// keep() it is kept again, if no other call's is; otherwise it is freed.
+// keep() it is kept again, if no other call's is and its bytes may be; otherwise
+// it is freed.  T::kept_bytes are the bytes counted for it while it is kept.
 template <class T, void (*Free)(T*)>
 class KeptState {
  public:
@@ -387,15 +397,20 @@ class KeptState {
     std::lock_guard<std::mutex> lk(mu_);
     std::swap(s_, kept_);
     if (!s_) s_ = new T();
+    drop_bytes(s_->device, s_->kept_bytes);
+    s_->kept_bytes = 0;
   }
   ~KeptState() { Free(s_); }
   KeptState(const KeptState&)            = delete;
   KeptState& operator=(const KeptState&) = delete;
   T& operator*() { return *s_; }
   T* operator->() { return s_; }
-  void keep() {
+  void keep(int device, uint64_t bytes) {
     std::lock_guard<std::mutex> lk(mu_);
-    if (!kept_) std::swap(s_, kept_);
+    if (kept_ || !keep_bytes(device, bytes)) return;
+    s_->device     = device;
+    s_->kept_bytes = bytes;
+    std::swap(s_, kept_);
   }
 
  private:

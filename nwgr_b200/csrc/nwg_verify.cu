@@ -482,6 +482,8 @@ namespace nwg {
 // levels took 4% longer.  One allocation for all arrays made a uniform graph of
 // 2^24 vertices 3% slower (12.5 ms against 12.9).
 struct VerifyWs {
+  int             device     = 0;
+  uint64_t        kept_bytes = 0;
   bool            ready   = false;
   bool            use_in  = false;    // csrs_transposed
   VerifyCounters* cnt     = nullptr;
@@ -495,6 +497,7 @@ struct VerifyWs {
 
 void verify_ws_free(VerifyWs* b) {
   if (!b) return;
+  drop_bytes(b->device, b->kept_bytes);
   if (b->s) cudaStreamSynchronize(b->s);
   cudaFree(b->depth);
   cudaFree(b->vis);
@@ -513,15 +516,19 @@ namespace {
 
 uint64_t queue_cap(const GraphDev* g) { return g->n / 4 + g->m / 512 + 1; }
 
+// Both queues, whose memory takes the pieces of long in-lists afterwards: in_m
+// / kVHub entries plus one per list of over kVHub, at most twice that.
+uint64_t queue_words(const GraphDev* g) {
+  return std::max<uint64_t>(2 * queue_cap(g), 2 * (g->in_m / kVHub) + 2);
+}
+
 int verify_ws_make(GraphDev* g, VerifyWs& b) {
   if (!b.s) NWG_CUDA_TRY(cudaStreamCreateWithFlags(&b.s, cudaStreamNonBlocking));
   const int rc = csrs_transposed(g, b.s, &b.use_in);
   if (rc) return rc;
-  // the pieces need m / kVHub entries plus one per list of over kVHub: at most twice that
-  const uint64_t q = std::max<uint64_t>(2 * queue_cap(g), 2 * (g->in_m / kVHub) + 2);
   if ((!b.depth && cudaMalloc(&b.depth, g->n * 4) != cudaSuccess) ||
       (!b.vis && cudaMalloc(&b.vis, 2 * ((g->n + 31) / 32) * 4) != cudaSuccess) ||
-      (!b.q && cudaMalloc(&b.q, q * 8) != cudaSuccess) ||
+      (!b.q && cudaMalloc(&b.q, queue_words(g) * 8) != cudaSuccess) ||
       (!b.cnt && cudaMalloc(&b.cnt, sizeof(VerifyCounters)) != cudaSuccess)) {
     cudaGetLastError();
     return set_error(NWG_ENOMEM, "verifier allocation failed (n=" + std::to_string(g->n) + ")");
@@ -620,7 +627,7 @@ int verify(GraphDev* g, uint32_t source, const uint32_t* parents_host, const uin
            nwg_verify_result* out) {
   KeptState<VerifyWs, verify_ws_free> b(g->kept_mu, g->verify_ws);
   const int rc = verify_on(g, *b, source, parents_host, parents_dev, out);
-  if (!rc) b.keep();
+  if (!rc) b.keep(g->device, 4 * g->n * (b->par ? 2 : 1) + g->n / 4 + queue_words(g) * 8);
   return rc;
 }
 
