@@ -337,8 +337,11 @@ int bfs_roots(GraphDev* g, const uint32_t* roots, uint64_t k, int alpha, int bet
   DeviceGuard                 dg(g->device);
   if (roots_by_block(g, k)) {
     const int rb = roots_run(g, roots, k, alpha, beta, parents_host);
-    if (status) std::fill(status, status + k, (int32_t)rb);
-    return rb;
+    if (rb != NWG_ENOMEM) {
+      if (status) std::fill(status, status + k, (int32_t)rb);
+      return rb;
+    }
+    // no room for the roots' rows and queues: one after another, in two workspaces
   }
   Workspace*                  w[2] = {nullptr, nullptr};
   int                         rc   = get_default_ws(g, &w[0]);
