@@ -394,7 +394,9 @@ int nwg_graph_write_nwbin(nwg_graph g, const char* path);
 
 /* Device BFSVerifier: the checks of nw::graph::BFSVerifier(g, g_t, source,
  * parent) (reference: include/nwgraph/algorithms/bfs.hpp:44-98) on the GPU,
- * for a parent array in host OR device memory (exactly one non-NULL).  Depths
+ * for a parent array in host OR device memory (exactly one non-NULL; a device
+ * array is read on a stream of the library's own, so the work that writes it
+ * must be complete).  Depths
  * come from a BFS over the out-graph written only for this check: it reads the
  * in-CSR to find them only where that is the out-CSR's transpose, which the
  * first call on a graph compares.  Its state (about 8 n + m / 32 bytes, and

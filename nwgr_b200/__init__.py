@@ -656,14 +656,19 @@ def betweenness(g: Graph, sources, normalize: bool = True, lanes: int = 0):
 
 def verify(g: Graph, root: int, parents) -> VerifyResult:
     """nw::graph::BFSVerifier on the GPU (bfs.hpp:44-98): parents is a host
-    uint32 array or a device tensor.  Returns the VerifyResult (valid, and
-    for an invalid array the lowest failing vertex and the reason)."""
+    uint32 array or a device tensor (read after the work queued on torch's
+    current stream).  Returns the VerifyResult (valid, and for an invalid array
+    the lowest failing vertex and the reason)."""
     r = VerifyResult()
     if isinstance(parents, np.ndarray):
         p = np.ascontiguousarray(parents, dtype=np.uint32)
         assert p.size >= g.n
         check(lib.nwg_verify(g.h, int(root), p.ctypes.data, None, C.byref(r)))
     else:
+        if getattr(parents, "is_cuda", False):  # the library reads it on a stream of its own
+            import torch
+
+            torch.cuda.current_stream(parents.device).synchronize()
         check(lib.nwg_verify(g.h, int(root), None, _ptr(parents), C.byref(r)))
     return r
 
