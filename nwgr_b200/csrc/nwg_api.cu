@@ -288,7 +288,7 @@ int bfs_sync(GraphDev* g, uint32_t root, int alpha, int beta, uint32_t* parents_
   if (rc) return rc;
   uint32_t* dst = parents_dev ? parents_dev : ws->parents;
   if (stats) NWG_CUDA_TRY(cudaEventRecord(ws->ev0, ws->stream));
-  if (blk_one_fits(g->n, g->m)) {
+  if (blk_one_fits(g->n, g->nzero, g->m)) {
     // the kernel writes what the host wants into pinned memory (RMAT-10: two
     // copies behind the traversal took longer than it)
     rc = ws_launch_to_host(ws, root, alpha, beta, dst, parents_host != nullptr, stats != nullptr, topdown_only);

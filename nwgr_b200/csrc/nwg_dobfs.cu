@@ -80,13 +80,28 @@ constexpr uint32_t kSoloPer    = kSoloCap / kThreads;  // list entries per threa
 constexpr int kBlkOneT   = 1024;
 constexpr int kBlkCopyT  = 512;
 constexpr int kBlkRootsT = 512;
-// A single traversal is one block's up to these sizes.  Device time of one
-// block against the whole grid (k_trav), B200: RMAT 2^10 21 / 64 us, 2^13
-// (204k edges) 32 / 72, uniform 2^13 (262k) 58 / 99, 2^14 (98k) 80 / 104,
-// grid 2^15 (131k) 330 / 412; past them the grid wins: uniform 2^14 (524k)
-// 118 / 64, 2^15 (197k) 130 / 115, grid 2^16 (262k) 548 / 458.
-constexpr uint64_t kBlkOneN = 1ull << 15;
-constexpr uint64_t kBlkOneM = 1ull << 18;
+// A single traversal is one block's up to these sizes (blk_one_fits): what one
+// SM does grows with the vertices that have edges, while the grid pays by the
+// level, so graphs of at most 6.5 entries a vertex, whose levels are many, stay
+// with the block for longer.  Device time of one block against the
+// whole grid (k_trav), B200, us:
+//   uniform, degree 4    2^14 70 / 117, 24,576 92 / 120, 2^15 120 / 124
+//   uniform, degree 6    2^14 66 / 93, 24,576 87 / 93, 28,672 90 / 109, 2^15 106 / 101
+//   uniform, degree 8    2^14 55 / 85, 24,576 85 / 86, 28,672 95 / 89, 2^15 112 / 90
+//   ... on 24,576 / 28,672 of 2^15 vertices 86 / 88, 110 / 91
+//   uniform, degree 10   18,432 77 / 87, 24,576 73 / 89
+//   uniform, degree 32   2^12 25 / 75, 2^13 47 / 81
+//   grid                 2^14 145 / 246, 24,576 192 / 259, 2^15 237 / 259
+//   RMAT (half isolated) 2^15, degree 4 / 6 / 8: 53 / 84, 54 / 73, 56 / 74
+//   path                 2^14 13,880 / 27,240
+//   star                 2^14 31 / 40, 24,576 38 / 42, 28,672 45 / 41, 2^15 49 / 41
+// With parents in host memory the block saves a copy and wins for longer:
+// degree 6 at 2^15 130 / 140, degree 8 at 28,672 117 / 128, at 2^15 135 / 130.
+// The star's loss is the price of the path's gain: neither count tells them
+// apart.
+constexpr uint64_t kBlkOneN      = 1ull << 15;
+constexpr uint64_t kBlkOneM      = 1ull << 18;
+constexpr uint64_t kBlkOneActive = 3ull << 13;  // vertices with edges, unless their entries are few
 
 __device__ __forceinline__ unsigned long long globaltimer() {
   unsigned long long t;
@@ -2598,10 +2613,10 @@ int ws_init(GraphDev* g, Workspace* ws) {
   NWG_CUDA_TRY(cudaStreamCreateWithFlags(&ws->stream, cudaStreamNonBlocking));
   NWG_CUDA_TRY(cudaEventCreate(&ws->ev0));
   NWG_CUDA_TRY(cudaEventCreate(&ws->ev1));
+  const uint64_t blk_n  = blk_one_fits(n, g->nzero, m) ? n : 0;  // one block's queue, and its parents for the host
   if (cudaMalloc(&ws->parents, std::max<uint64_t>(n, 4) * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&ws->V, 3ull * std::max<uint32_t>(nwords, 1) * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&ws->qbuf, std::max<uint64_t>(2 * qs_cap * sizeof(uint32_t), blk_one_fits(n, m) ? n * sizeof(BlkEnt) : 0)) !=
-          cudaSuccess ||
+      cudaMalloc(&ws->qbuf, std::max<uint64_t>(2 * qs_cap * sizeof(uint32_t), blk_n * sizeof(BlkEnt))) != cudaSuccess ||
       cudaMalloc(&ws->cbuf, 2ull * qc_cap * sizeof(uint64_t)) != cudaSuccess ||
       cudaMalloc(&ws->hubbuf, 2ull * hub_cap * sizeof(HubRec)) != cudaSuccess ||
       cudaMalloc(&ws->ctrl, sizeof(Ctrl)) != cudaSuccess) {
@@ -2609,8 +2624,7 @@ int ws_init(GraphDev* g, Workspace* ws) {
     return set_error(NWG_ENOMEM, "workspace allocation failed (n=" + std::to_string(n) + ")");
   }
   // beside the control block, a small graph's parents for the host
-  const uint64_t host_n = blk_one_fits(n, m) ? n : 0;
-  NWG_CUDA_TRY(cudaMallocHost(&ws->ctrl_host, sizeof(Ctrl) + host_n * sizeof(uint32_t)));
+  NWG_CUDA_TRY(cudaMallocHost(&ws->ctrl_host, sizeof(Ctrl) + blk_n * sizeof(uint32_t)));
   ws->parents_host = reinterpret_cast<uint32_t*>(ws->ctrl_host + 1);
   NWG_CUDA_TRY(cudaMemset(ws->ctrl, 0, sizeof(Ctrl)));
 
@@ -2738,7 +2752,12 @@ static int blk_prepare() {
 
 static BlkGraph blk_graph(const DobfsParams& P) { return BlkGraph{P.off, P.col, P.in_off, P.in_col, P.Z, P.n, P.m}; }
 
-bool blk_one_fits(uint64_t n, uint64_t m) { return n <= kBlkOneN && m <= kBlkOneM; }
+// Whether a single traversal is one block's; nzero vertices have no in-edges
+// (0 where that is not known).
+bool blk_one_fits(uint64_t n, uint64_t nzero, uint64_t m) {
+  const uint64_t active = n - std::min(n, nzero);
+  return n <= kBlkOneN && m <= kBlkOneM && (active <= kBlkOneActive || 2 * m <= 13 * active);
+}
 
 static int blk_one_launch(const BlkGraph& g, uint32_t root, int alpha, int beta, uint32_t* parents, BlkEnt* q,
                           Ctrl* ctrl, bool topdown_only, const BlkHost& host, cudaStream_t stream) {
@@ -2788,7 +2807,7 @@ int ws_launch(Workspace* ws, uint32_t root, int alpha, int beta, uint32_t* paren
   if (alpha <= 0 || beta <= 0) return set_error(NWG_EINVAL, "alpha and beta must be positive");
   uint32_t  r = root, a = (uint32_t)alpha, b = (uint32_t)beta, td = topdown_only ? 1u : 0u;
   uint32_t* par    = parents ? parents : ws->parents;
-  if (blk_one_fits(g->n, g->m)) {
+  if (blk_one_fits(g->n, g->nzero, g->m)) {
     const int rc = blk_one_launch(blk_graph(ws->params), root, alpha, beta, par,
                                   reinterpret_cast<BlkEnt*>(ws->qbuf), ws->ctrl, topdown_only, BlkHost{}, stream);
     if (rc) return rc;
@@ -2808,7 +2827,7 @@ int ws_launch(Workspace* ws, uint32_t root, int alpha, int beta, uint32_t* paren
 int run_traversal(const DobfsParams& params, int sm_count, uint32_t root, int alpha, int beta, uint32_t* parents,
                   void* q, cudaStream_t stream) {
   DobfsParams P = params;
-  if (blk_one_fits(P.n, P.m)) {
+  if (blk_one_fits(P.n, P.nzero, P.m)) {
     BlkGraph g = blk_graph(P);
     g.Z        = nullptr;  // not built
     return blk_one_launch(g, root, alpha, beta, parents, static_cast<BlkEnt*>(q), P.ctrl, false, BlkHost{}, stream);

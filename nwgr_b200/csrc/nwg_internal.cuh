@@ -342,7 +342,7 @@ int    ragged_block_threads(const RaggedDev* r, double max_weight, double sum_we
 double blk_weight(uint64_t n, uint64_t m);
 uint64_t ragged_scratch_bytes(const RaggedDev* r, bool any_big, uint32_t blocks_per_sm, int threads);
 bool ragged_by_block(uint64_t n, uint64_t m);
-bool blk_one_fits(uint64_t n, uint64_t m);
+bool blk_one_fits(uint64_t n, uint64_t nzero, uint64_t m);
 bool roots_by_block(const GraphDev* g, uint64_t k);
 int  roots_run(GraphDev* g, const uint32_t* roots, uint64_t k, int alpha, int beta, uint32_t* parents_host);
 void roots_pool_free(struct RootsPool* p);
