@@ -73,6 +73,7 @@ typedef struct {
    * one action per iteration but the last; a persistent small-frontier
    * action covers several steps in one launch) */
   uint32_t kernel_launches;
+  uint32_t offer_steps; /* steps whose edges offered parents instead of claiming their targets */
 } nwg_bfs_stats;
 
 /* Library version string. */

@@ -749,6 +749,7 @@ __device__ __forceinline__ void init_step(const DobfsParams& p, uint32_t root, u
     c.prev_small  = 0;
     c.mark_ok     = 0;
     c.b2q_then_td = 0;
+    c.offer_steps = 0;
     const uint64_t cap = 2 * n + 64;
     c.max_steps = cap > 0xFFFFFF00ull ? 0xFFFFFF00u : (uint32_t)cap;
   }
@@ -913,6 +914,7 @@ __device__ __forceinline__ uint32_t mark_offers(const DobfsParams& p, const Ctrl
 __device__ __forceinline__ uint32_t mark_setup(const DobfsParams& p, CtrlHdr& c, uint64_t front,
                                                uint64_t front_edges) {
   c.mark_offer = mark_offers(p, c, front, front_edges);
+  c.offer_steps += c.mark_offer;
   c.bu_push   = 0;
   c.acc_awake = 0;
   c.acc_scout = 0;
@@ -925,6 +927,7 @@ __device__ __forceinline__ uint32_t mark_setup(const DobfsParams& p, CtrlHdr& c,
 __device__ __forceinline__ uint32_t mark_td_setup(const DobfsParams& p, CtrlHdr& c, uint64_t front,
                                                   uint64_t front_edges) {
   c.mark_offer = mark_offers(p, c, front, front_edges);
+  c.offer_steps += c.mark_offer;
   c.acc_awake = 0;
   c.acc_scout = 0;
   c.bm        = 1;
@@ -2406,6 +2409,7 @@ __global__ void __launch_bounds__(T)
     c.bu_steps     = r.bu_steps;
     c.b2q_steps    = r.b2q_steps;
     c.reached      = r.reached;
+    c.offer_steps  = 0;
     c.trace_len    = ntr;
     ctrl->kernels  = 1;
     ctrl->decides  = 0;
@@ -3028,6 +3032,7 @@ void fill_stats(const Ctrl& c, nwg_bfs_stats* s) {
     s->trace_end_ns[i]   = c.trace_end_ns[i];
   }
   s->first_decide_ns = c.t_first_decide;
+  s->offer_steps     = c.h.offer_steps;
 }
 
 // Builds the in-degree-zero bitmap Z, its population (g->nzero; the bits

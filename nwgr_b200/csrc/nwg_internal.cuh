@@ -90,7 +90,7 @@ struct alignas(16) CtrlHdr {
   uint32_t mark_ok;      // kActBUMark / kActTDMark may be chosen (set by the persistent kernel in its copies)
   uint32_t b2q_then_td;  // the bitmap -> queue pass rebuilds the queue of a marking top-down step
   uint32_t mark_offer;   // the marking step offers parents instead of claiming
-  uint32_t pad_[1];
+  uint32_t offer_steps;  // such steps so far
 };
 static_assert(sizeof(CtrlHdr) % 16 == 0, "the header is copied in 16-byte pieces");
 
