@@ -19,7 +19,9 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+from array import array
 from dataclasses import dataclass, field
+from itertools import chain
 
 import numpy as np
 
@@ -419,11 +421,21 @@ class RaggedBatch:
         import torch
 
         k = len(items)
-        table = np.array(items, np.int64).reshape(k, 5)
-        arr = table.astype(np.uint32)  # rows of RaggedItem (alpha and beta keep their bits)
-        # sizes of valid items only: the C layer rejects bad ones with a message
-        g = table[:, 0]
-        total = int(self.n[g[(g >= 0) & (g < self.num_graphs)]].sum())
+        table = None
+        try:
+            if set(map(len, items)) == {5}:
+                table = np.frombuffer(array("q", chain.from_iterable(items)), np.int64).reshape(k, 5)
+        except (TypeError, ValueError, OverflowError, RuntimeError):
+            pass
+        # total: sizes of valid items only, the C layer rejects bad ones with a message
+        if table is not None:
+            arr = table.astype(np.uint32)  # rows of RaggedItem (alpha and beta keep their bits)
+            g = table[:, 0]
+            total = int(self.n[g[(g >= 0) & (g < self.num_graphs)]].sum())
+        else:  # fields that are no integers, but may be to int()
+            arr = np.array([(int(g), int(r), int(a), int(b), int(w)) for g, r, a, b, w in items], object).reshape(k, 5)
+            arr = (arr & 0xFFFFFFFF).astype(np.uint32)
+            total = sum(int(self.n[g]) for g, *_ in items if 0 <= int(g) < self.num_graphs)
         if parents_dev is None:
             parents_dev = torch.empty(max(total, 1), dtype=torch.int32, device="cuda")
         offs = np.zeros(k, np.uint64)
