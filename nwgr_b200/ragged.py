@@ -8,17 +8,18 @@ persistent launch, parameters from an autotuner cached per graph-shape class.
 
 Graph-shape class: (floor(log2 n), round(log2 average degree)) -- the two
 quantities that set a traversal's level count, frontier sizes and hub
-weight.  Per class the tuner chooses the top-down degree threshold
-(warp_min: vertices at or above it are expanded in 256-edge chunks by a
-whole warp) and the direction switch points alpha, beta (the reference's
-defaults are 15 and 18; any choice gives the same depths, only the work
-changes); per batch it chooses the resident blocks per SM of the persistent
-launch.  Choices are timed on the device (CUDA events of the persistent
-launch) over a sample of each class's items.
+weight.  Per class the tuner chooses the direction switch points alpha, beta
+(the reference's defaults are 15 and 18; any choice gives the same depths, only
+the work changes) and, where a class has graphs of more than 2^19 vertices, the
+top-down degree threshold (warp_min: vertices at or above it are expanded in
+256-edge chunks by a whole warp; the kernel of the smaller graphs has none).
+Per batch it chooses the resident blocks per SM of the persistent launch; that
+kernel runs at most two.  Choices are timed on the device (CUDA events of the
+persistent launch) over a sample of each class's items.
 
 Cache: JSON at $NWG_AUTOTUNE_CACHE, else $XDG_CACHE_HOME/nwgr_b200/autotune.json
-(~/.cache when XDG_CACHE_HOME is unset), keyed by GPU name and library
-version.  Tuning results belong to the machine that measured them, so the
+(~/.cache when XDG_CACHE_HOME is unset), keyed by GPU name, library version
+and KERNELS.  Tuning results belong to the machine that measured them, so the
 package ships none: a class the cache lacks is tuned on first use.
 """
 from __future__ import annotations
@@ -39,10 +40,14 @@ def default_cache_path() -> str:
     return os.path.join(base, "nwgr_b200", "autotune.json")
 
 
+KERNELS = "kernels 2"  # raised when a change of the ragged kernels outdates tuned values
 WARP_MIN = (32, 64, 128)
 ALPHA = (15, 60)
 BETA = (18, 36)
 BLOCKS_PER_SM = (1, 2, 3)
+# Graphs of at most these sizes are traversed with their bitmaps in shared
+# memory, by at most two blocks per SM and without warp_min.
+BLOCK_MAX_N, BLOCK_MAX_M = 1 << 19, (1 << 31) - 1
 
 
 def shape_class(n: int, m: int) -> str:
@@ -64,7 +69,11 @@ def _device_key() -> str:
         name = torch.cuda.get_device_name(0)
     except Exception:
         name = "unknown"
-    return f"{name}|{version()}"
+    return f"{name}|{version()}|{KERNELS}"
+
+
+def _past_block(n: int, m: int) -> bool:
+    return n > BLOCK_MAX_N or m > BLOCK_MAX_M
 
 
 class Autotuner:
@@ -116,7 +125,7 @@ class Autotuner:
             pick = gs[:: max(1, len(gs) // sample)][:sample]
             base = [(g, int(r)) for g in pick for r in roots_by_graph[g]]
             best, best_t = ClassParams(), float("inf")
-            for wm in WARP_MIN:
+            for wm in WARP_MIN if any(_past_block(*graph_mn[g]) for g in gs) else (best.warp_min,):
                 for a in ALPHA:
                     for b in BETA:
                         t = self._time(batch, [(g, r, a, b, wm) for g, r in base], 2)
@@ -127,7 +136,8 @@ class Autotuner:
         bps = self.entry.get("blocks_per_sm")
         if bps is None or force:
             items = self.items(graph_mn, roots_by_graph, out)
-            times = {b: self._time(batch, items, b, 2) for b in BLOCKS_PER_SM}
+            sweep = BLOCKS_PER_SM if any(_past_block(n, m) for n, m in graph_mn) else BLOCKS_PER_SM[:2]
+            times = {b: self._time(batch, items, b, 2) for b in sweep}
             bps = min(times, key=times.get)
             self.entry["blocks_per_sm"] = bps
         self.save()
