@@ -523,10 +523,9 @@ __device__ __forceinline__ void flush_block(const DobfsParams& p, const StepView
 // atomic, never a wrong claim), then the unvisited ones are claimed with
 // atomicOr (all issued before any result is used).  A claim's winner writes parents[v] = u (the reference's CAS
 // winner) and is buffered; scout and the next queue are updated when the
-// buffer is flushed.  In a marking step (kMark; sv.mark) the winner instead
-// sets its bit in sv.mark and counts itself in `nbig`, which such a step
-// adds to the awake count; a marking top-down step (sv.mark_deg) adds its
-// out-degree to `scout` as well.  All 32 lanes must call.
+// buffer is flushed.  In a marking step (kMark == kClaim) the winner only
+// writes its parent; mark_collect counts the discoveries afterwards.  All 32
+// lanes must call.
 template <bool kDefer, int kMark = kQueue>
 __device__ __forceinline__ void visit_batch(const DobfsParams& p, const StepView& sv, const uint32_t (&u)[kVisit],
                                             const uint32_t (&v)[kVisit], uint32_t valid, TdWarp& tw, uint32_t& wcnt,
@@ -902,7 +901,9 @@ __device__ __forceinline__ bool mark_td(const DobfsParams& p, const CtrlHdr& c, 
 // claims, 203 with an atomic for every edge), it has at most 2.5 out-edges per
 // vertex of the graph, and at most a quarter of the graph is visited.  Uniform
 // 2^24's step over 30M edges: 458 us with claims, 405 with an atomic for every
-// edge, 340 with offers.
+// edge, 340 with offers.  Over uniform graphs of degree 2 to 64 and RMAT graphs
+// of degree 4 to 64, 2^16 to 2^24 vertices, no traversal takes longer on the
+// device than it did with claims alone.
 __device__ __forceinline__ uint32_t mark_offers(const DobfsParams& p, const CtrlHdr& c, uint64_t front,
                                                 uint64_t front_edges) {
   return front_edges <= 2 * p.avg_deg * front && 2 * front_edges <= 5 * p.active && front_edges >= p.n / 2 &&
@@ -1222,8 +1223,9 @@ __device__ __forceinline__ void td_step(const DobfsParams& p, const StepView& sv
 // up for each discovery as it is claimed costs two scattered L2 accesses
 // beside the claim and the parent: uniform 2^24's step of 13M discoveries
 // took 609 us that way, 458 us with this pass; RMAT-24's of 3M 168 and 152.
-// Steps without claims (each edge to an unvisited vertex stores its parent,
-// this pass reads the parents) took 440 and 196 us: not kept.
+// Storing a parent for each edge to an unvisited vertex, without a claim, and
+// reading the parents in this pass took 440 and 196 us; steps that store one
+// for every edge into a buffer of their own are offer_collect's.
 // Not inlined: its registers would add to the step functions' spills.
 __device__ __noinline__ void mark_collect(const uint32_t* V, uint32_t* mark, uint64_t n, const uint16_t* deg16,
                                           const uint64_t* off, bool deg, unsigned long long* awake_out,
@@ -1407,16 +1409,11 @@ __device__ __forceinline__ bool grid_barrier(const DobfsParams& p, unsigned nblo
   return s_ok != 0;
 }
 
-// k_td_loop: the small-frontier branch.  A persistent cooperative kernel of
-// kSmallBlocks blocks runs consecutive top-down steps, each followed by a
-// grid barrier and the decision (block 0), while the frontier stays small
-// and the direction stays top-down; it then leaves the next decision for
-// the graph's decide node (pre_decided).  Long, thin traversals (grids,
-// roads) thus pay a barrier per level instead of two kernel launches.
-// Writes the chunk entries of the hub records the level deferred (queue
+// Writes the chunk entries of the hub records that a level deferred (queue
 // buffer qi): a warp per record, grid-strided, so the writes come from every
-// SM.  Runs after the level's barrier, beside the decision; the next barrier
-// (or the kernel's end) orders them before the next level reads the queue.
+// SM.  Runs after the level's barrier: in k_trav after the decision, if the
+// step that it chose reads the queue, here beside it.  The next barrier (or the
+// kernel's end) orders the entries before that step.
 __device__ __forceinline__ void expand_hubs(const DobfsParams& p, uint32_t qi, uint64_t nhub, uint32_t block,
                                             uint32_t nblocks) {
   const HubRec* rec = p.hubrec[qi];
@@ -1436,6 +1433,12 @@ __device__ __forceinline__ void expand_hubs(const DobfsParams& p, uint32_t qi, u
   }
 }
 
+// k_td_loop: the small-frontier branch.  A persistent cooperative kernel of
+// kSmallBlocks blocks runs consecutive top-down steps, each followed by a
+// grid barrier and the decision (block 0), while the frontier stays small
+// and the direction stays top-down; it then leaves the next decision for
+// the host's next k_decide (pre_decided).  Long, thin traversals (grids,
+// roads) thus pay a barrier per level instead of two kernel launches.
 __global__ void __launch_bounds__(kThreads) k_td_loop(DobfsParams p) {
   __shared__ TdWarp   s_tw[kWarps];
   __shared__ uint32_t s_next;
@@ -2255,7 +2258,8 @@ __global__ void __launch_bounds__(kThreads, kTravPerSm)
           offer_collect(p.V, s_c.bm ? p.C0 : p.C1, p.qs[s_c.cur ^ 1u], s_c.parents, p.n, p.deg16, p.off,
                         s_next == kActTDMark, &acc->awake, &acc->scout);
         else
-        mark_collect(p.V, s_c.bm ? p.C0 : p.C1, p.n, p.deg16, p.off, s_next == kActTDMark, &acc->awake, &acc->scout);
+          mark_collect(p.V, s_c.bm ? p.C0 : p.C1, p.n, p.deg16, p.off, s_next == kActTDMark, &acc->awake,
+                       &acc->scout);
       } else {
         td_step<true>(p, sv, sm.td.tw, blockIdx.x, gridDim.x);
       }
@@ -2888,8 +2892,9 @@ static uint32_t roots_slots(const GraphDev* g) {
 
 // A block takes about 20 us and 4 ns per weighted vertex (kBlkRootsT
 // threads) for a root, side by side with the launch's others; the grid 60 us
-// or more for each root, one after another (its traversals of graphs of up
-// to 2^19 vertices: 61-590 us).
+// or more for each root with its copy, one after another.  Over grids, uniform
+// and RMAT graphs and stars of 2^12 to 2^19 vertices and 2 to 300 roots, no
+// call took over 3% longer than with the grid alone.
 bool roots_by_block(const GraphDev* g, uint64_t k) {
   if (g->n > kBlkMaxN || g->m >= kBlkMaxM || k < 2) return false;
   const double waves = std::ceil((double)k / roots_slots(g));
