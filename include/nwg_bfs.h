@@ -345,7 +345,9 @@ int nwg_server_run_trace(nwg_server s, uint32_t count, const uint32_t* graph, co
  * looks the array's device address up and keeps it for the life of the
  * process: do not use this entry point on a device across cudaDeviceReset,
  * which unloads the module that holds the array.  The traversal runs on
- * `stream` (a cudaStream_t, NULL = legacy default stream) and the call
+ * `stream` (a cudaStream_t, NULL = legacy default stream), on all but small
+ * graphs as a cooperative launch that waits until its blocks fit on the GPU
+ * beside what is running, and the call
  * synchronises that stream, so it must not be called while the stream is
  * being captured into a CUDA graph; it returns when the traversal is
  * complete. */
