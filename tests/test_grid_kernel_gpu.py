@@ -10,6 +10,7 @@ import pytest
 
 from oracle import graphgen as gg
 from test_dobfs_gpu import _fan_bipartite, _path_star
+from test_pull_batch_gpu import _sparse
 
 pytestmark = pytest.mark.gpu
 NULL = 0xFFFFFFFF
@@ -147,6 +148,16 @@ def test_offering_steps_run(nwg, port, n, deg, directed):
         assert port.verify(*csr[:2], r, host[i + 1:i + 1 + n], *csr[2:])
         assert np.all(host[: i + 1] == 7) and np.all(host[i + 1 + n:] == 7)
     assert offers >= 2
+    g.release()
+
+
+@pytest.mark.parametrize("n,deg,directed", [(40000, 4, False), (65535, 4, True), (131072, 2, False)])
+def test_traces_of_sparse_pulls_are_whole(nwg, port, n, deg, directed):
+    csr = _sparse(n, deg, n // 2000, n, directed)
+    csr = csr[: 4 if directed else 2]
+    g = nwg.Graph.from_csr(*csr)
+    assert sum(_check(nwg, port, g, csr, r, *ab).bu_steps for r in map(int, gg.roots(csr[0], 3, seed=deg))
+               for ab in ((15, 18), (100, 1000))) > 0
     g.release()
 
 
